@@ -29,9 +29,11 @@ enum : int {
 
 // The update kernel's point-by-point walks read a candidate point's
 // coordinates and its sin / 1 - cos offsets as whole 16-byte records when
-// d <= kPackDims: pack_w(d) float4 of coordinates, pack_s(d) float4 of the
+// packed_dims(d): pack_w(d) float4 of coordinates, pack_s(d) float4 of the
 // 2d offsets, zero-padded.
 constexpr int kPackDims = 8;
+// d = 7 has no kernels of its own: the generic ones keep sd and md.
+__host__ __device__ constexpr bool packed_dims(int d) { return d <= kPackDims && d != 7; }
 __host__ __device__ constexpr int pack_w(int d) { return (d + 3) / 4; }
 __host__ __device__ constexpr int pack_s(int d) { return (2 * d + 3) / 4; }
 

@@ -156,7 +156,7 @@ size_t layout_work(const Geom& g, int max_iter, char* base, Work& w, float** xin
     };
     add((void**)&w.X, 4 * d * ns);
     add((void**)&w.Xn, 4 * d * ns);
-    const bool packed = d <= kPackDims;
+    const bool packed = packed_dims(d);
     add((void**)&w.sd, packed ? 0 : 4 * d * ns);
     add((void**)&w.md, packed ? 0 : 4 * d * ns);
     add((void**)&w.xp, packed ? 16 * (size_t)pack_w(d) * ns : 0);
