@@ -17,6 +17,7 @@
 namespace egg {
 
 constexpr int kScanSmallTiles = 64;  // radix digit scan: one block per instance up to this many tiles
+constexpr int kWideBatchPer = 16;    // points per block of the wide update (d > 4) in a batch
 constexpr int kMaxBatch = 1024;      // instances of one batched call
 
 // launch shapes: how many blocks a kernel uses for one instance
@@ -33,7 +34,7 @@ enum Shape : int {
     kShapeCapOuter,    // min(ceil(n_outer / 64), 148 * 8): 8 outer cells per warp
     kShapeFix,         // min(ceil(ceil(n / 32) / 8), 148 * 8)
     kShapeCapN256L,    // min(ceil(n / 256), 148 * 16)
-    kShapeN64,         // ceil(n / 64)
+    kShapeWide,        // ceil(n / kWideBatchPer): kWideBatchPer points a block (d > 4)
     kShapeCount
 };
 
@@ -55,7 +56,7 @@ __host__ __device__ inline int shape_blocks(int shape, const Geom& g) {
         case kShapeCapOuter: return cap(cdiv(g.n_outer, 64) > 0 ? cdiv(g.n_outer, 64) : 1, 148 * 8);
         case kShapeFix: return cap(cdiv(cdiv(g.n, 32), 8), 148 * 8);
         case kShapeCapN256L: return cap(cdiv(g.n, 256), 148 * 16);
-        case kShapeN64: return cdiv(g.n, 64);
+        case kShapeWide: return cdiv(g.n, kWideBatchPer);
         default: return 1;
     }
 }

@@ -232,7 +232,7 @@ __global__ void k_batch_results(const Work* works, int count, int* out) {
 // host side
 // ---------------------------------------------------------------------------
 struct Config {
-    int update_threads = 128;
+    int update_threads = 256;
     int occ = 8;
     int order = 1;
     bool operator<(const Config& o) const {
@@ -318,7 +318,7 @@ struct Plan {
     int* d_boff_all = nullptr;
     int* d_active_all = nullptr;
     int* d_nact_all = nullptr;
-    int* d_loop = nullptr;            // [2 + groups]: iterations, any active, sort openings per group
+    int* d_loop = nullptr;            // [2 + 2 groups]: iterations, any active, sort and tile-order openings per group
     int* d_results = nullptr;
     unsigned long long* d_loop_stamps = nullptr;
     float* d_in = nullptr;            // staged host inputs
@@ -415,11 +415,15 @@ void set_tables(Plan& P, const Config& c) {
             bt->update_threads = c.update_threads;
             bt->max_passes = 0;
             bt->max_table_k = 0;
+            bt->tile = false;
+            bt->bytes = true;
             for (int s = 0; s < kShapeCount; s++) bt->total[s] = 0;
             for (int i = 0; i < P.count; i++) {
                 if (P.geoms[i].d != gr.d) continue;
                 bt->max_passes = std::max(bt->max_passes, plan_count(P.geoms[i]));
                 bt->max_table_k = std::max(bt->max_table_k, P.geoms[i].table_k);
+                bt->tile = bt->tile || tile_capable(P.geoms[i]);
+                bt->bytes = bt->bytes && byte_keys(P.geoms[i]);
                 for (int s = 0; s < kShapeCount; s++) bt->total[s] += shape_blocks(s, P.geoms[i]);
             }
         }
@@ -433,15 +437,17 @@ void set_tables(Plan& P, const Config& c) {
 }
 
 // one iteration of group k's instances.  Parts, in order: 0 = grid check,
-// 1 = grid sort, 2 = cell sums, need, update, 3 = extra check; in the loop
-// graph parts 1 and 3 sit behind conditional nodes (gated: the extra
-// check's gate did the stage stamp and count).  -1 = all four, ungated.
+// 1 = grid sort, 4 = tile order of the new grids, 2 = cell sums, need,
+// update, 3 = extra check; in the loop graph parts 1, 4 (inside part 1's
+// body) and 3 sit behind conditional nodes (gated: the extra check's gate
+// did the stage stamp and count).  -1 = all, ungated.
 void enqueue_group(Plan& P, int k, cudaStream_t st, int part = -1) {
     Group& gr = P.groups[k];
     const Exec ex = batched(gr.act, gr.d);
     const bool all = part < 0;
     if (all || part == 0) launch_build_check(ex, st, false);  // the control kernel cleared the changed words
     if (all || part == 1) launch_build_sort(ex, st);
+    if (all || part == 4) launch_tile_order(ex, st);
     if (all || part == 2) {
         launch_cell_sums(ex, st);
         launch_need(ex, st);
@@ -480,6 +486,8 @@ std::vector<char> graph_key(const Plan& P) {
         put(g.act.total, sizeof(g.act.total));
         put(&g.act.max_passes, sizeof(int));
         put(&g.act.max_table_k, sizeof(int));
+        put(&g.act.tile, sizeof(bool));
+        put(&g.act.bytes, sizeof(bool));
     }
     return k;
 }
@@ -564,15 +572,20 @@ cudaGraphExec_t get_graph(State& S, Plan& P, const Config& c) {
                 if (r == cudaSuccess && last && !*last) r = cudaErrorUnknown;
                 return r;
             };
-            // an IF node after `dep` whose body is `fn`; the node -> *node
-            auto cond = [&](cudaGraphConditionalHandle hc, cudaGraphNode_t dep, cudaGraphNode_t* node, auto&& fn) {
+            // an IF node in `into` after `dep` whose body `fill` captures; the node -> *node
+            auto cond = [&](cudaGraph_t into, cudaGraphConditionalHandle hc, cudaGraphNode_t dep, cudaGraphNode_t* node,
+                            auto&& fill) {
                 cudaGraphNodeParams xp = {cudaGraphNodeTypeConditional};
                 xp.conditional.handle = hc;
                 xp.conditional.type = cudaGraphCondTypeIf;
                 xp.conditional.size = 1;
-                cudaError_t r = cudaGraphAddNode(node, gbody, &dep, 1, &xp);
-                if (r == cudaSuccess) r = seg(xp.conditional.phGraph_out[0], nullptr, nullptr, fn);
+                cudaError_t r = cudaGraphAddNode(node, into, &dep, 1, &xp);
+                if (r == cudaSuccess) r = fill(xp.conditional.phGraph_out[0]);
                 return r;
+            };
+            auto cond_leaf = [&](cudaGraph_t into, cudaGraphConditionalHandle hc, cudaGraphNode_t dep,
+                                 cudaGraphNode_t* node, auto&& fn) {
+                return cond(into, hc, dep, node, [&](cudaGraph_t b) { return seg(b, nullptr, nullptr, fn); });
             };
             cudaGraphConditionalHandle hsort, hx;
             e = cudaGraphConditionalHandleCreate(&hsort, gbody, 0, 0);
@@ -583,13 +596,28 @@ cudaGraphExec_t get_graph(State& S, Plan& P, const Config& c) {
                     launch_batch_gate_sort(gex, hsort, P.d_loop + 2 + k, S.st);
                 });
             cudaGraphNode_t ifs_sort = nullptr, ifs_x = nullptr;
-            if (e == cudaSuccess) e = cond(hsort, prev, &ifs_sort, [&] { enqueue_group(P, k, S.st, 1); });
+            // sort body: [sort, gate] -> IF(some instance wants a tile order) [tile order]
+            if (e == cudaSuccess)
+                e = cond(gbody, hsort, prev, &ifs_sort, [&](cudaGraph_t sb) {
+                    if (!gex.tile) return seg(sb, nullptr, nullptr, [&] { enqueue_group(P, k, S.st, 1); });
+                    cudaGraphConditionalHandle ht;
+                    cudaGraphNode_t last = nullptr, it_node = nullptr;
+                    cudaError_t r = cudaGraphConditionalHandleCreate(&ht, sb, 0, 0);
+                    if (r == cudaSuccess)
+                        r = seg(sb, nullptr, &last, [&] {
+                            enqueue_group(P, k, S.st, 1);
+                            launch_batch_gate_tile(gex, ht, P.d_loop + 2 + G + k, S.st);
+                        });
+                    if (r == cudaSuccess)
+                        r = cond_leaf(sb, ht, last, &it_node, [&] { enqueue_group(P, k, S.st, 4); });
+                    return r;
+                });
             if (e == cudaSuccess)
                 e = seg(gbody, ifs_sort, &prev, [&] {
                     enqueue_group(P, k, S.st, 2);
                     launch_batch_gate_extra(gex, hx, S.st);
                 });
-            if (e == cudaSuccess) e = cond(hx, prev, &ifs_x, [&] { enqueue_group(P, k, S.st, 3); });
+            if (e == cudaSuccess) e = cond_leaf(gbody, hx, prev, &ifs_x, [&] { enqueue_group(P, k, S.st, 3); });
             if (!ok && e == cudaSuccess) e = cudaErrorUnknown;
         }
         if (e == cudaSuccess) {
@@ -649,6 +677,8 @@ void make_plan(State& S, Plan& P, egg_batch_item* items, int count, const egg_op
             throw ArgError{EGG_ERR_ARG, "item " + std::to_string(i) + ": x and labels must not be NULL"};
         try {
             P.geoms[i] = make_geom(it.n, it.d, it.eps);
+            P.geoms[i].tile_min = kTileMinBatchN;
+            P.geoms[i].point_walk = it.d > 4;
         } catch (ArgError& e) {
             e.msg = "item " + std::to_string(i) + ": " + e.msg;
             throw;
@@ -713,7 +743,7 @@ void make_plan(State& S, Plan& P, egg_batch_item* items, int count, const egg_op
     const size_t o_boff_all = reserve(4 * tab);
     const size_t o_act_all = reserve(4 * (size_t)G * P.cap);
     const size_t o_nact_all = reserve(4 * G);
-    const size_t o_loop = reserve(4 * (2 + (size_t)G));
+    const size_t o_loop = reserve(4 * (2 + 2 * (size_t)G));
     const size_t o_res = reserve(4 * 5 * (size_t)count);
     const size_t o_ls = reserve(8 * ((size_t)P.max_iter + 2));
     const size_t o_in = reserve(4 * P.in_floats);
@@ -806,15 +836,16 @@ int enqueue_prologue(State& S, Plan& P, int max_iter) {
         kb_load<<<ex.blocks(kShapeCapN256L, 256), 256, 0, S.st>>>(ex.args(kShapeCapN256L));
         launches++;
     }
-    EGG_CHECK(cudaMemsetAsync(P.d_loop, 0, 4 * (2 + P.groups.size()), S.st));
+    EGG_CHECK(cudaMemsetAsync(P.d_loop, 0, 4 * (2 + 2 * P.groups.size()), S.st));
     k_batch_ctl<<<1, 1024, 0, S.st>>>(ctl_args(P), 0, 0, 0);
     return launches + 1;
 }
 
 // kernels of one group's iteration: grid check, sort (radix passes, 4
-// tables), cell sums (2), need, update, extra check (3)
+// tables), tile order (keys, 3 per pass), cell sums (2), need, update, extra check (3)
 int sort_launches(const Group& gr) { return 3 * gr.act.max_passes + 4; }
-int group_launches(const Group& gr) { return 1 + sort_launches(gr) + 2 + 1 + 1 + 3; }
+int tile_launches(const Group& gr) { return gr.act.tile ? 1 + 3 * tile_passes(gr.d) : 0; }
+int group_launches(const Group& gr) { return 1 + sort_launches(gr) + tile_launches(gr) + 2 + 1 + 1 + 3; }
 
 // Kernels of the loop graph: gate and control every iteration, and each
 // group's kernels in the iterations where it had active instances (the
@@ -830,8 +861,9 @@ long long loop_launches(const Plan& P, int loop_iters, const std::vector<int>& r
         const Group& gr = P.groups[k];
         int m = 0;
         for (int pos = gr.begin; pos < gr.end; pos++) m = std::max(m, res[5 * (size_t)pos]);
-        l += (long long)m * (group_launches(gr) - 3 - sort_launches(gr) + 2) +
-             (long long)opened[k] * sort_launches(gr) + 3LL * (gr.end - gr.begin);
+        l += (long long)m * (group_launches(gr) - 3 - sort_launches(gr) - tile_launches(gr) + 2) +
+             (long long)opened[k] * (sort_launches(gr) + (tile_launches(gr) ? 1 : 0)) +
+             (long long)opened[P.groups.size() + k] * tile_launches(gr) + 3LL * (gr.end - gr.begin);
     }
     return l;
 }
@@ -877,16 +909,20 @@ Config autotune(State& S, Plan& P) {
     time_trial(S, P, best);  // warm-up: graph instantiation, caches
     auto trial2 = [&](const Config& c) { return std::min(time_trial(S, P, c), time_trial(S, P, c)); };
     float tb = trial2(best);
+    // the trials see the first iterations only, where nearly every point is
+    // recomputed; blocks of 256 cost least in the many that follow (one sweep's
+    // last 500 iterations: 36.6 ms, 40 with 128 and 46 with 64), so the others
+    // have to be 5% ahead
     auto consider = [&](Config c) {
         const float t = trial2(c);
-        if (t < tb) {
+        if (t < tb * (c.update_threads != best.update_threads ? 0.95f : 1.0f)) {
             tb = t;
             best = c;
         }
     };
     consider(Config{best.update_threads, best.occ, 1 - best.order});
     const Config b1 = best;
-    for (int ut : {64, 256}) consider(Config{ut, b1.occ, b1.order});
+    consider(Config{128, b1.occ, b1.order});
     const Config b2 = best;
     for (int occ : {4, 16}) consider(Config{b2.update_threads, occ, b2.order});
     return best;
@@ -977,7 +1013,7 @@ int run_batch(egg_batch_item* items, int count, const egg_opts* opts_in, egg_bat
     launches++;
     const size_t out_b = 4 * P.out_ints;
     if (out_b) EGG_CHECK(cudaMemcpyAsync(S.h_pinned, P.d_out, out_b, cudaMemcpyDeviceToHost, S.st));
-    const size_t nloop = 2 + P.groups.size();
+    const size_t nloop = 2 + 2 * P.groups.size();
     std::vector<int> res(5 * (size_t)count + nloop);
     EGG_CHECK(cudaMemcpyAsync(res.data(), P.d_results, 4 * 5 * (size_t)count, cudaMemcpyDeviceToHost, S.st));
     EGG_CHECK(cudaMemcpyAsync(res.data() + 5 * (size_t)count, P.d_loop, 4 * nloop, cudaMemcpyDeviceToHost, S.st));

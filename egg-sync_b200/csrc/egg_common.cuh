@@ -20,10 +20,17 @@ constexpr int kSortTile = 2048;     // points per radix-sort tile (2048: 489 blo
 constexpr int kSortThreads = 256;
 constexpr int kHeadsBlock = 1024;   // points per block in the cell-boundary scan
 
+// Dimensions and sizes whose updates may run in tile order (egg_grid.cu).
+// Below 16,384 points 32 to a warp leave most of the chip idle: there every
+// point gets a warp (10k x 2D, a run's updates: 0.71 -> 0.24 ms; in tile order
+// 0.51, and 0.28 for the sorts).  A batch sorts all its instances in one go,
+// and its small ones want the order too.
+constexpr int kTileMinN = 16384, kTileMinBatchN = 1024;
+__host__ __device__ constexpr bool tile_dims(int d) { return d >= 2 && d <= 4; }
+
 // Status word bits set by kernels (read by the host after the run).
 enum : int {
     kErrNonFinite = 1,       // input holds NaN/Inf
-    kErrTable = 2,           // a cell offset fell outside the sin/cos table
     kErrStencil = 4,
 };
 
@@ -36,6 +43,18 @@ constexpr int kPackDims = 8;
 __host__ __device__ constexpr bool packed_dims(int d) { return d <= kPackDims && d != 7; }
 __host__ __device__ constexpr int pack_w(int d) { return (d + 3) / 4; }
 __host__ __device__ constexpr int pack_s(int d) { return (2 * d + 3) / 4; }
+
+// A cell's sums and its tight box are records of whole 16-byte words, one
+// per cell: sum_w(d) floats hold sum sin(delta) [d] then sum (1 - cos) [d]
+// (the order of smp), box_w(d) floats each hold the box's lower and upper
+// corner.  A visit reads a record with one 16-byte load per four values
+// where dimension-major arrays took one 4-byte load per value, and a lane
+// walking on its own touches one or two sectors per record instead of one
+// per dimension.
+__host__ __device__ constexpr int sum_w(int d) { return 4 * pack_s(d); }
+__host__ __device__ constexpr int box_w(int d) { return 4 * pack_w(d); }
+__host__ __device__ constexpr int group_w(int d) { return sum_w(d) + 2 * box_w(d); }
+constexpr int kByteDims = 16;  // cells of d in (4, 16] with width <= 256: one byte per dimension, 16 bytes a cell
 
 // Per-instance geometry, exactly as the reference computes it
 // (src/algorithms/EGG_SynC.cu:1249-1260, 1430, 563, 779, 1045).
@@ -62,6 +81,8 @@ struct Geom {
     int order_mode;    // 0 = no order parameter, 1 = final only, 2 = every iteration
     float lam;         // order-parameter threshold of stop rule 1
     int zblk;          // incremental update: cells of dimension od per block (1 block when od == d)
+    int tile_min;      // points from which d = 2, 3, 4 may run in tile order
+    int point_walk;    // the update gives every point a warp of its own
     int nzb;           // ... number of blocks (<= 64: one bit each)
     int wpow[32];      // width^l for l < od
 };
@@ -78,8 +99,7 @@ struct Work {
     float4* smp;       // [ns][pack_s(d)] sin(delta) then 1 - cos(delta), packed per point (d <= kPackDims)
     float* qlo;        // [d][ns] eps/2-ball extremes (extra check)
     float* qhi;        // [d][ns]
-    float* ulo;        // [d][ns] per cell: union of its points' eps/2-ball extremes
-    float* uhi;        // [d][ns]
+    float* ubox;       // [ns][2 * box_w(d)] per cell: union of its points' eps/2-ball extremes
     int* orig;         // [ns]   original index of sorted point i
     int* orig_tmp;     // [ns]
     int* perm;         // [ns]   radix sort output: new position -> previous position
@@ -92,10 +112,9 @@ struct Work {
     int* cell_dims;    // [d][ns]
     unsigned long long* cell_key;  // [ns] the cell's dims packed 16 bits each (d <= 4): one load per box test
     int* cell_outer;   // [ns]
-    float* css;        // [d][ns] sum sin(delta) per cell
-    float* csm;        // [d][ns] sum (1 - cos(delta)) per cell
-    float* cbmin;      // [d][ns] tight bounding box of the cell's points
-    float* cbmax;      // [d][ns]
+    unsigned char* cell_bytes;     // [ns][16] the cell's dims as bytes (4 < d <= 16, width <= 256; else nullptr)
+    float* csum;       // [ns][sum_w(d)] per cell: sum sin(delta) [d], sum (1 - cos(delta)) [d]
+    float* cbox;       // [ns][2 * box_w(d)] tight bounding box of the cell's points: lower, then upper corner
     int* outer_begin;  // [n_outer + 1]
     unsigned long long* colmask;  // [n_outer] per outer cell: the blocks of zblk cells of dimension od holding a cell
     // scratch for scans / sorts
@@ -103,7 +122,7 @@ struct Work {
     int* digit_total;  // [256]
     int* block_sums;   // [blocks]
     double* wpart;     // [(2d values + 2d bbox) * 2 * warps] warp partials for spanning cells
-    float* gpart;      // the same records in FP32: the 32-point groups of spanning cells
+    float* gpart;      // [2 * warps][group_w(d)] in FP32: sums, then box, of the 32-point groups of spanning cells
     // stencils (host-built tables)
     int* st_delta;     // [3][st_cap] linear outer-id offset
     signed char* st_off;  // [3][st_cap * od] per-dimension offsets
@@ -156,6 +175,11 @@ enum : int {
     kCtrlFullUpdate = 14, // recompute every point in every iteration
     kCtrlSpanCount = 15,  // cells over 2-3 warps listed in span_list by the cell-sums kernel
     kCtrlBigCount = 16,   // cells over 4 or more warps listed in big_list
+    kCtrlTileWant = 18,   // this rebuild's grid gets a tile order (most points were recomputed lately)
+    kCtrlTiled = 19,      // perm holds the tile order of the current grid
+    kCtrlTileBase = 20,   // kCtrlComputed and kCtrlIter at the last rebuild
+    kCtrlTileIter = 21,
+    kCtrlTileSorts = 22,  // tile orders made (statistics)
     kCtrlLamReached = 17, // the order parameter's lower bound reached lambda this iteration
     kCtrlWords = 32,      // size of the control-word array
 };
@@ -252,23 +276,64 @@ __device__ __forceinline__ float near_gap(float x, float lo, float hi) {
 }
 
 // Squared distances from x to the nearest and to the farthest point of the
-// tight bounding box [lo, hi] of a cell's points, accumulated with the same
-// fused operation order as dist_step.  Every float step is monotone, so for
-// each point q of the cell near2 <= dist2(x, q) <= far2 holds exactly as the
-// kernels compute dist2: near2 > T proves no point passes "dist2 <= T", and
-// far2 <= T proves all of them do.
-__device__ __forceinline__ void tight_box_dist2(const float* x, const float* __restrict__ lo,
-                                                const float* __restrict__ hi, size_t stride, int d, float& near2,
+// tight bounding box [lo, hi] of a cell's points (a box record: lower corner,
+// then upper corner), accumulated with the same fused operation order as
+// dist_step.  Every float step is monotone, so for each point q of the cell
+// near2 <= dist2(x, q) <= far2 holds exactly as the kernels compute dist2:
+// near2 > T proves no point passes "dist2 <= T", and far2 <= T proves all of
+// them do.
+template <int D>
+__device__ __forceinline__ void tight_box_dist2(const float* x, const float* __restrict__ box, int d, float& near2,
                                                 float& far2) {
     float a2 = 0.f, b2 = 0.f;
-    for (int l = 0; l < d; l++) {
-        const float L = __ldg(lo + (size_t)l * stride), H = __ldg(hi + (size_t)l * stride);
-        const float a = near_gap(x[l], L, H), b = far_gap(x[l], L, H);
-        a2 = __fmaf_rn(a, a, a2);
-        b2 = __fmaf_rn(b, b, b2);
+    if constexpr (D > 0) {
+        const float4* b = reinterpret_cast<const float4*>(box);
+#pragma unroll
+        for (int k = 0; k < pack_w(D); k++) {
+            const float4 L4 = __ldg(b + k), H4 = __ldg(b + pack_w(D) + k);
+            const float L[4] = {L4.x, L4.y, L4.z, L4.w}, H[4] = {H4.x, H4.y, H4.z, H4.w};
+#pragma unroll
+            for (int l = 4 * k; l < 4 * k + 4 && l < D; l++) {
+                const float a = near_gap(x[l], L[l & 3], H[l & 3]), c = far_gap(x[l], L[l & 3], H[l & 3]);
+                a2 = __fmaf_rn(a, a, a2);
+                b2 = __fmaf_rn(c, c, b2);
+            }
+        }
+    } else {
+        for (int l = 0; l < d; l++) {
+            const float L = __ldg(box + l), H = __ldg(box + box_w(d) + l);
+            const float a = near_gap(x[l], L, H), c = far_gap(x[l], L, H);
+            a2 = __fmaf_rn(a, a, a2);
+            b2 = __fmaf_rn(c, c, b2);
+        }
     }
     near2 = a2;
     far2 = b2;
+}
+
+// a cell's box record, and the record of a 32-point group (rec 0 = the
+// segment holding the warp's lane 0, rec 1 = the segment holding lane 31)
+template <int D>
+__device__ __forceinline__ const float* cell_box(const Work& w, int c, int d) {
+    return w.cbox + (size_t)c * (2 * box_w(D > 0 ? D : d));
+}
+template <int D>
+__device__ __forceinline__ const float* cell_sum(const Work& w, int c, int d) {
+    return w.csum + (size_t)c * sum_w(D > 0 ? D : d);
+}
+template <int D>
+__device__ __forceinline__ float* group_rec(const Work& w, int warp, int rec, int d) {
+    return w.gpart + ((size_t)warp * 2 + rec) * group_w(D > 0 ? D : d);
+}
+
+// cells of this geometry carry byte keys (Work::cell_bytes)
+__host__ __device__ inline bool byte_keys(const Geom& g) { return g.d > 4 && g.d <= kByteDims && g.width <= 256; }
+
+// the tile order's curve has 8 bits per dimension, an 8-bit sort pass each
+constexpr int kTileBits = 8;
+__host__ __device__ constexpr int tile_passes(int d) { return d; }
+__host__ __device__ inline bool tile_capable(const Geom& g) {
+    return tile_dims(g.d) && g.od >= 1 && g.n >= g.tile_min;
 }
 
 // index of a warp-partial record: ((field * d + l) * 2 + rec) * warps + warp,

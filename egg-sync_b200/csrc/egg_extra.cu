@@ -100,9 +100,10 @@ __device__ bool mbr_exact(const Geom& g, const Work& w, int qi, const float* xp)
 // them (the cell's first) stands for all.  Near convergence nearly every
 // cell is such a collapsed cluster (1M x 3D: 41,646 of 41,660 final cells,
 // holding all but 44 points).
-__device__ __forceinline__ bool cell_degenerate(const Geom& g, const Work& w, int c, int d) {
+__device__ __forceinline__ bool cell_degenerate(const Work& w, int c, int d) {
+    const float* b = cell_box<0>(w, c, d);
     for (int l = 0; l < d; l++)
-        if (__ldg(w.cbmin + (size_t)l * g.ns + c) != __ldg(w.cbmax + (size_t)l * g.ns + c)) return false;
+        if (__ldg(b + l) != __ldg(b + box_w(d) + l)) return false;
     return true;
 }
 
@@ -122,7 +123,7 @@ __device__ __forceinline__ void ball_bbox_body(const Geom& g, const Work& w, int
     for (int i = bx * blockDim.x + threadIdx.x; i < g.n; i += gx * blockDim.x) {
         // in a collapsed cell only the first point's extremes are read
         const int ci = w.cell_of[i];
-        if (i != w.cell_start[ci] && cell_degenerate(g, w, ci, d)) continue;
+        if (i != w.cell_start[ci] && cell_degenerate(w, ci, d)) continue;
         float xq[DM], lo[DM], hi[DM];
         int gq[DM];
         int obase = 0;
@@ -139,12 +140,13 @@ __device__ __forceinline__ void ball_bbox_body(const Geom& g, const Work& w, int
             if (!(sm2 <= g.t_half)) return true;
             // none / all of the cell's points inside the eps/2 ball?
             float near2, far2;
-            tight_box_dist2(xq, w.cbmin + c, w.cbmax + c, g.ns, d, near2, far2);
+            const float* box = cell_box<D>(w, c, d);
+            tight_box_dist2<D>(xq, box, d, near2, far2);
             if (near2 > g.t_half) return true;
             if (far2 <= g.t_half) {
                 for (int l = 0; l < d; l++) {
-                    lo[l] = fminf(lo[l], __ldg(w.cbmin + (size_t)l * g.ns + c));
-                    hi[l] = fmaxf(hi[l], __ldg(w.cbmax + (size_t)l * g.ns + c));
+                    lo[l] = fminf(lo[l], __ldg(box + l));
+                    hi[l] = fmaxf(hi[l], __ldg(box + box_w(d) + l));
                 }
                 return true;
             }
@@ -179,7 +181,7 @@ __device__ __forceinline__ void cell_ballbox_body(const Geom& g, const Work& w, 
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     for (int c = bx * wpb + (threadIdx.x >> 5); c < M; c += gx * wpb) {
         const int qb = w.cell_start[c], qe = w.cell_start[c + 1];
-        const bool deg = cell_degenerate(g, w, c, g.d);
+        const bool deg = cell_degenerate(w, c, g.d);
         for (int l = 0; l < g.d; l++) {
             float lo, hi;
             if (deg) {
@@ -199,8 +201,9 @@ __device__ __forceinline__ void cell_ballbox_body(const Geom& g, const Work& w, 
                 }
             }
             if (lane == 0) {
-                w.ulo[(size_t)l * g.ns + c] = lo;
-                w.uhi[(size_t)l * g.ns + c] = hi;
+                float* u = w.ubox + (size_t)c * (2 * box_w(g.d));
+                u[l] = lo;
+                u[box_w(g.d) + l] = hi;
             }
         }
     }
@@ -217,7 +220,7 @@ __device__ __forceinline__ void annulus_body(const Geom& g, const Work& w, int b
         // a point of a collapsed cell finds what the cell's first point finds
         const int cp = w.cell_of[i];
         const int pb = w.cell_start[cp];
-        const bool pdeg = cell_degenerate(g, w, cp, d);
+        const bool pdeg = cell_degenerate(w, cp, d);
         if (pdeg && i != pb) continue;
         const int pw = pdeg ? w.cell_start[cp + 1] - pb : 1;  // points it stands for (pair count)
         float xp[DM];
@@ -238,14 +241,14 @@ __device__ __forceinline__ void annulus_body(const Geom& g, const Work& w, int b
             const bool fully = lg2 <= g.t_eps;
             if (!included || fully) return true;
             float near2, far2;
-            tight_box_dist2(xp, w.cbmin + c, w.cbmax + c, g.ns, d, near2, far2);
+            tight_box_dist2<D>(xp, cell_box<D>(w, c, d), d, near2, far2);
             if (near2 > g.t_extra || far2 <= g.t_eps) return true;
             float lb2, ub2;
-            tight_box_dist2(xp, w.ulo + c, w.uhi + c, g.ns, d, lb2, ub2);
+            tight_box_dist2<D>(xp, w.ubox + (size_t)c * (2 * box_w(d)), d, lb2, ub2);
             if (lb2 > g.t_eps) return true;  // no pair of this cell can have its MBR within eps
             const int qb = __ldg(w.cell_start + c), qe = __ldg(w.cell_start + c + 1);
             // a collapsed cell: its first point decides for all of them
-            const bool qdeg = cell_degenerate(g, w, c, d);
+            const bool qdeg = cell_degenerate(w, c, d);
             const int qend = qdeg ? qb + 1 : qe;
             for (int q = qb; q < qend; q++) {
                 float d2 = 0.f;
@@ -367,6 +370,28 @@ __global__ void __launch_bounds__(1024) k_batch_gate_sort(const Work* __restrict
 
 void launch_batch_gate_sort(const Exec& ex, cudaGraphConditionalHandle h, int* opened, cudaStream_t st) {
     k_batch_gate_sort<<<1, 1024, 0, st>>>(ex.bt->works, ex.bt->active, ex.bt->nact, opened, h);
+}
+
+// The same for the tile order, after the sort: open when a rebuilt grid of
+// the group wants one.
+__global__ void __launch_bounds__(1024) k_batch_gate_tile(const Work* __restrict__ works,
+                                                          const int* __restrict__ active, const int* __restrict__ nact,
+                                                          int* __restrict__ opened, cudaGraphConditionalHandle h) {
+    const int na = *nact;
+    int want = 0;
+    for (int t = threadIdx.x; t < na; t += blockDim.x) {
+        const int* c = works[active[t]].ctrl;
+        want |= c[kCtrlChanged] != 0 && c[kCtrlTileWant] != 0;
+    }
+    const int any = __syncthreads_or(want);
+    if (threadIdx.x == 0) {
+        if (any) *opened += 1;
+        cudaGraphSetConditional(h, any ? 1u : 0u);
+    }
+}
+
+void launch_batch_gate_tile(const Exec& ex, cudaGraphConditionalHandle h, int* opened, cudaStream_t st) {
+    k_batch_gate_tile<<<1, 1024, 0, st>>>(ex.bt->works, ex.bt->active, ex.bt->nact, opened, h);
 }
 
 // The kernels return at once unless the update left the flag at 1; the

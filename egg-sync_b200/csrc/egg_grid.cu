@@ -300,7 +300,6 @@ __device__ __forceinline__ void onekey_keys_body(const Geom& g, const Work& w, i
 }
 
 __device__ __forceinline__ void onekey_hist_body(const Geom& g, const Work& w, int p, int bx) {
-    EGG_SKIP_IF_UNCHANGED(w.ctrl);
     __shared__ int h[256];
     const int tiles = (g.n + kSortTile - 1) / kSortTile;
     const unsigned* kin = w.skey[p & 1];
@@ -313,13 +312,11 @@ __device__ __forceinline__ void onekey_hist_body(const Geom& g, const Work& w, i
 }
 
 // stable scatter of one tile of (key, previous position) pairs
-__device__ __forceinline__ void onekey_scatter_body(const Geom& g, const Work& w, int p, int bx) {
-    EGG_SKIP_IF_UNCHANGED(w.ctrl);
+__device__ __forceinline__ void onekey_scatter_body(const Geom& g, const Work& w, int p, int P, int bx) {
     constexpr int kWarps = kSortThreads / 32;
     __shared__ int base[256];
     __shared__ int run[256];
     __shared__ int wcnt[kWarps][256];
-    const int P = onekey_passes(g);
     const int tiles = (g.n + kSortTile - 1) / kSortTile;
     const unsigned* kin = w.skey[p & 1];
     unsigned* kout = w.skey[(p + 1) & 1];
@@ -401,6 +398,82 @@ __device__ __forceinline__ void gather_heads_body(const Geom& g, const Work& w, 
     if (threadIdx.x == 0) w.block_sums[bx] = total;
 }
 
+// ---------------------------------------------------------------------------
+// Tile order (d = 2, 3, 4): the points along a Hilbert curve of their cells.
+// Storage order is column-major, so 32 consecutive points of a sparse column
+// lie dozens of cells apart in dimension od and a warp of them cannot share
+// its candidates; along the curve a warp's points fill a few neighbouring
+// cells, and the update walks their joint candidates in lockstep.  The order
+// only groups the update's threads: no result depends on it.
+// ---------------------------------------------------------------------------
+// Making the order costs a sort of n short keys; the update gets it back
+// when it recomputes most points.  The first iteration recomputes all; later
+// the mean per iteration since the last rebuild stands for the next one.
+__device__ __forceinline__ bool tile_order_pays(const Geom& g, const Work& w) {
+    if (!tile_capable(g) || w.skey[0] == nullptr) return false;
+    const int it = w.ctrl[kCtrlIter], done = w.ctrl[kCtrlComputed];
+    const long long its = it - w.ctrl[kCtrlTileIter], cmp = (unsigned)done - (unsigned)w.ctrl[kCtrlTileBase];
+    w.ctrl[kCtrlTileIter] = it;
+    w.ctrl[kCtrlTileBase] = done;
+    return w.ctrl[kCtrlForce] != 0 || 2 * cmp >= (long long)g.n * its;
+}
+
+#define EGG_SKIP_IF_UNTILED(ctrl) \
+    if ((ctrl)[kCtrlChanged] == 0 || (ctrl)[kCtrlTileWant] == 0) return;
+
+// Hilbert index of cell coordinates v of b bits each (J. Skilling,
+// "Programming the Hilbert curve", AIP Conf. Proc. 707, 2004)
+template <int D>
+__device__ __forceinline__ unsigned hilbert_index(unsigned* v, int b) {
+    for (unsigned q = 1u << (b - 1); q > 1; q >>= 1) {
+        const unsigned p = q - 1;
+#pragma unroll
+        for (int l = 0; l < D; l++) {
+            if (v[l] & q) {
+                v[0] ^= p;
+            } else {
+                const unsigned t = (v[0] ^ v[l]) & p;
+                v[0] ^= t;
+                v[l] ^= t;
+            }
+        }
+    }
+#pragma unroll
+    for (int l = 1; l < D; l++) v[l] ^= v[l - 1];
+    unsigned t = 0;
+    for (unsigned q = 1u << (b - 1); q > 1; q >>= 1)
+        if (v[D - 1] & q) t ^= q - 1;
+#pragma unroll
+    for (int l = 0; l < D; l++) v[l] ^= t;
+    unsigned key = 0;
+    for (int k = b - 1; k >= 0; k--)
+#pragma unroll
+        for (int l = 0; l < D; l++) key = (key << 1) | ((v[l] >> k) & 1u);
+    return key;
+}
+
+// the payload starts where an even number of passes ends in perm
+__device__ __forceinline__ int* tile_payload(const Geom& g, const Work& w, int p) {
+    return ((tile_passes(g.d) - p) & 1) ? w.perm_tmp : w.perm;
+}
+
+template <int D>
+__device__ __forceinline__ void tile_keys_body(const Geom& g, const Work& w, int bx, int gx) {
+    EGG_SKIP_IF_UNTILED(w.ctrl);
+    constexpr int b = kTileBits;
+    const int sh = max(0, 32 - __clz(g.width - 1) - b);  // cells wider than the key's bits share a code
+    int* v0 = tile_payload(g, w, 0);
+    if (bx == 0 && threadIdx.x == 0) w.ctrl[kCtrlTileSorts] += 1;
+    for (int i = bx * blockDim.x + threadIdx.x; i < g.n; i += gx * blockDim.x) {
+        const int c = w.cell_of[i];
+        unsigned v[D];
+#pragma unroll
+        for (int l = 0; l < D; l++) v[l] = (unsigned)__ldg(w.cell_dims + (size_t)l * g.ns + c) >> sh;
+        w.skey[0][i] = hilbert_index<D>(v, b);
+        v0[i] = i;
+    }
+}
+
 // single-block exclusive scan of the per-block head counts; M = total
 __device__ __forceinline__ void scan_block_sums_body(const Geom& g, const Work& w) {
     EGG_SKIP_IF_UNCHANGED(w.ctrl);
@@ -422,6 +495,9 @@ __device__ __forceinline__ void scan_block_sums_body(const Geom& g, const Work& 
         w.ctrl[kCtrlM] = total;
         w.ctrl[kCtrlGridValid] = 1;
         w.ctrl[kCtrlBuilds] += 1;
+        // the tile order goes with the grid; a new one is made where it pays
+        w.ctrl[kCtrlTiled] = 0;
+        w.ctrl[kCtrlTileWant] = tile_order_pays(g, w) ? 1 : 0;
         // the spanning-cell lists describe the grid: rebuilt with it
         w.ctrl[kCtrlSpanCount] = 0;
         w.ctrl[kCtrlBigCount] = 0;
@@ -460,6 +536,12 @@ __device__ __forceinline__ void heads_finalize_body(const Geom& g, const Work& w
             }
             w.cell_outer[c] = outer;
             if (d <= 4 && w.cell_key) w.cell_key[c] = key;
+            if (w.cell_bytes) {
+                unsigned b[kByteDims / 4] = {};
+                for (int l = 0; l < d; l++)
+                    b[l >> 2] |= (unsigned)cell_dim(w.X[(size_t)l * g.ns + i], g) << (8 * (l & 3));
+                *reinterpret_cast<uint4*>(w.cell_bytes + (size_t)c * kByteDims) = make_uint4(b[0], b[1], b[2], b[3]);
+            }
         }
         if (i == g.n - 1) w.cell_start[c + 1] = g.n;
     }
@@ -492,6 +574,17 @@ __device__ __forceinline__ void outer_ranges_body(const Geom& g, const Work& w, 
                 atomicOr(w.colmask + oc, ((unsigned long long)hi << 32) | lo);
         }
     }
+}
+
+// dimension l of a cell's sum and box records
+template <int D>
+__device__ __forceinline__ void put_cell(const Work& w, int c, int l, int d, float ss, float sm, float mn, float mx) {
+    float* cs = w.csum + (size_t)c * sum_w(D > 0 ? D : d);
+    float* cb = w.cbox + (size_t)c * (2 * box_w(D > 0 ? D : d));
+    cs[l] = ss;
+    cs[(D > 0 ? D : d) + l] = sm;
+    cb[l] = mn;
+    cb[box_w(D > 0 ? D : d) + l] = mx;
 }
 
 // ---------------------------------------------------------------------------
@@ -579,10 +672,7 @@ __device__ __forceinline__ void cell_sums_body(const Geom& g, const Work& w, int
             }
         }
         if (complete) {
-            w.css[(size_t)l * g.ns + c] = __fadd_rn(vs.hi, vs.lo);
-            w.csm[(size_t)l * g.ns + c] = __fadd_rn(vm.hi, vm.lo);
-            w.cbmin[(size_t)l * g.ns + c] = mn;
-            w.cbmax[(size_t)l * g.ns + c] = mx;
+            put_cell<D>(w, c, l, d, __fadd_rn(vs.hi, vs.lo), __fadd_rn(vm.hi, vm.lo), mn, mx);
         } else if (seg_end) {
             // partial of a cell spanning several warps: rec 0 = segment holding
             // lane 0 (continues from the previous warp), rec 1 = segment holding
@@ -598,10 +688,11 @@ __device__ __forceinline__ void cell_sums_body(const Geom& g, const Work& w, int
                 w.wpart[wp_idx(1, l, d, rec, nw, warp)] = Mm;
                 w.wpart[wp_idx(2, l, d, rec, nw, warp)] = mn;
                 w.wpart[wp_idx(3, l, d, rec, nw, warp)] = mx;
-                w.gpart[wp_idx(0, l, d, rec, nw, warp)] = Sf;
-                w.gpart[wp_idx(1, l, d, rec, nw, warp)] = Mf;
-                w.gpart[wp_idx(2, l, d, rec, nw, warp)] = mn;
-                w.gpart[wp_idx(3, l, d, rec, nw, warp)] = mx;
+                float* gr = group_rec<D>(w, warp, rec, d);
+                gr[l] = Sf;
+                gr[d + l] = Mf;
+                gr[sum_w(d) + l] = mn;
+                gr[sum_w(d) + box_w(d) + l] = mx;
             }
         }
     }
@@ -677,10 +768,7 @@ __device__ void combine_big(const Geom& g, const Work& w, int c, int wh, int wt,
                 mx[l] = fmax(mx[l], __shfl_xor_sync(0xffffffffu, mx[l], o));
             }
             if (lane == 0) {
-                w.css[(size_t)l * g.ns + c] = (float)S[l];
-                w.csm[(size_t)l * g.ns + c] = (float)Mm[l];
-                w.cbmin[(size_t)l * g.ns + c] = (float)mn[l];
-                w.cbmax[(size_t)l * g.ns + c] = (float)mx[l];
+                put_cell<D>(w, c, l, d, (float)S[l], (float)Mm[l], (float)mn[l], (float)mx[l]);
             }
         }
     } else {
@@ -701,10 +789,7 @@ __device__ void combine_big(const Geom& g, const Work& w, int c, int wh, int wt,
                 mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
             }
             if (lane == 0) {
-                w.css[(size_t)l * g.ns + c] = (float)S;
-                w.csm[(size_t)l * g.ns + c] = (float)Mm;
-                w.cbmin[(size_t)l * g.ns + c] = (float)mn;
-                w.cbmax[(size_t)l * g.ns + c] = (float)mx;
+                put_cell<D>(w, c, l, d, (float)S, (float)Mm, (float)mn, (float)mx);
             }
         }
     }
@@ -742,7 +827,8 @@ __device__ void combine_big_field(const Geom& g, const Work& w, int c, int wh, i
                 acc[l] = f < 2 ? acc[l] + v[u][l] : (f == 2 ? fmin(acc[l], v[u][l]) : fmax(acc[l], v[u][l]));
         }
     }
-    float* out = f == 0 ? w.css : (f == 1 ? w.csm : (f == 2 ? w.cbmin : w.cbmax));
+    // the field's place in the cell's sum or box record
+    float* out = f < 2 ? w.csum + (size_t)c * sum_w(D) + f * D : w.cbox + (size_t)c * (2 * box_w(D)) + (f - 2) * box_w(D);
 #pragma unroll
     for (int l = 0; l < D; l++) {
         double a = acc[l];
@@ -751,7 +837,7 @@ __device__ void combine_big_field(const Geom& g, const Work& w, int c, int wh, i
             const double b = __shfl_xor_sync(0xffffffffu, a, o);
             a = f < 2 ? a + b : (f == 2 ? fmin(a, b) : fmax(a, b));
         }
-        if (lane == 0) out[(size_t)l * g.ns + c] = (float)a;
+        if (lane == 0) out[l] = (float)a;
     }
 }
 
@@ -770,6 +856,10 @@ __device__ __forceinline__ void cell_sums_fix_body(const Geom& g, const Work& w,
     const bool rebuilt = w.ctrl[kCtrlChanged] != 0;
     const int it = w.ctrl[kCtrlIter];
     const int big = w.ctrl[kCtrlBigCount];
+    // an update in tile order, or with a warp per point, marks the storage
+    // warps of the points it moves: the last update's marks are read by now
+    if (g.point_walk || w.ctrl[kCtrlTiled] != 0)
+        for (int k = bx * blockDim.x + threadIdx.x; k < nw; k += gx * blockDim.x) w.warp_moved[k] = 0;
     const int warps = (gx * blockDim.x) >> 5;
     if constexpr (D > 0) {
         // a warp per (cell, field)
@@ -801,10 +891,7 @@ __device__ __forceinline__ void cell_sums_fix_body(const Geom& g, const Work& w,
                 mn = fmin(mn, w.wpart[wp_idx(2, l, d, rec, nw, k)]);
                 mx = fmax(mx, w.wpart[wp_idx(3, l, d, rec, nw, k)]);
             }
-            w.css[(size_t)l * g.ns + c] = (float)S;
-            w.csm[(size_t)l * g.ns + c] = (float)Mm;
-            w.cbmin[(size_t)l * g.ns + c] = (float)mn;
-            w.cbmax[(size_t)l * g.ns + c] = (float)mx;
+            put_cell<D>(w, c, l, d, (float)S, (float)Mm, (float)mn, (float)mx);
         }
     }
 }
@@ -900,10 +987,50 @@ __global__ void __launch_bounds__(kSortThreads) kb_radix_scatter(BatchArgs B, in
 }
 __global__ void __launch_bounds__(256) k_onekey_keys(Geom g, Work w) { onekey_keys_body(g, w, blockIdx.x, gridDim.x); }
 __global__ void __launch_bounds__(kSortThreads) k_onekey_hist(Geom g, Work w, int p) {
+    EGG_SKIP_IF_UNCHANGED(w.ctrl);
     onekey_hist_body(g, w, p, blockIdx.x);
 }
 __global__ void __launch_bounds__(kSortThreads) k_onekey_scatter(Geom g, Work w, int p) {
-    onekey_scatter_body(g, w, p, blockIdx.x);
+    EGG_SKIP_IF_UNCHANGED(w.ctrl);
+    onekey_scatter_body(g, w, p, onekey_passes(g), blockIdx.x);
+}
+// tile order: the same passes over the Hilbert codes
+template <int D>
+__global__ void __launch_bounds__(256) k_tile_keys(Geom g, Work w) { tile_keys_body<D>(g, w, blockIdx.x, gridDim.x); }
+template <int D>
+__global__ void __launch_bounds__(256) kb_tile_keys(BatchArgs B) {
+    batch_for(B, [&](const Geom& g, const Work& w, int bx, int gx) { tile_keys_body<D>(g, w, bx, gx); });
+}
+__device__ __forceinline__ void tile_hist_body(const Geom& g, const Work& w, int p, int bx) {
+    EGG_SKIP_IF_UNTILED(w.ctrl);
+    if (p < tile_passes(g.d)) onekey_hist_body(g, w, p, bx);
+}
+__device__ __forceinline__ void tile_scan_body(const Geom& g, const Work& w, int p, int bx) {
+    EGG_SKIP_IF_UNTILED(w.ctrl);
+    if (p < tile_passes(g.d)) radix_scan_body(g, w, bx);
+}
+__device__ __forceinline__ void tile_scatter_body(const Geom& g, const Work& w, int p, int bx) {
+    EGG_SKIP_IF_UNTILED(w.ctrl);
+    const int P = tile_passes(g.d);
+    if (p >= P) return;
+    onekey_scatter_body(g, w, p, P, bx);
+    if (p == P - 1 && bx == 0 && threadIdx.x == 0) w.ctrl[kCtrlTiled] = 1;
+}
+__global__ void __launch_bounds__(kSortThreads) k_tile_hist(Geom g, Work w, int p) {
+    tile_hist_body(g, w, p, blockIdx.x);
+}
+__global__ void __launch_bounds__(256) k_tile_scan(Geom g, Work w, int p) { tile_scan_body(g, w, p, blockIdx.x); }
+__global__ void __launch_bounds__(kSortThreads) k_tile_scatter(Geom g, Work w, int p) {
+    tile_scatter_body(g, w, p, blockIdx.x);
+}
+__global__ void __launch_bounds__(kSortThreads) kb_tile_hist(BatchArgs B, int p) {
+    batch_for(B, [&](const Geom& g, const Work& w, int bx, int) { tile_hist_body(g, w, p, bx); });
+}
+__global__ void __launch_bounds__(256) kb_tile_scan(BatchArgs B, int p) {
+    batch_for(B, [&](const Geom& g, const Work& w, int bx, int) { tile_scan_body(g, w, p, bx); });
+}
+__global__ void __launch_bounds__(kSortThreads) kb_tile_scatter(BatchArgs B, int p) {
+    batch_for(B, [&](const Geom& g, const Work& w, int bx, int) { tile_scatter_body(g, w, p, bx); });
 }
 template <int D>
 __global__ void __launch_bounds__(kHeadsBlock) k_gather_heads(Geom g, Work w) {
@@ -1035,6 +1162,28 @@ void launch_build_sort(const Exec& ex, cudaStream_t st) {
     EGG_GO(ex, kShapeOne, 1024, st, scan_block_sums);
     EGG_GO_D(ex, kShapeN1024, kHeadsBlock, st, heads_finalize);
     EGG_GO(ex, kShapeOuter, 256, st, outer_ranges);
+}
+
+// the tile order of a rebuilt grid; every kernel returns at once where the
+// rebuild found it does not pay
+void launch_tile_order(const Exec& ex, cudaStream_t st) {
+    if (!ex.tile) return;
+    const int blocks = ex.blocks(kShapeCapN256L, 256), P = tile_passes(ex.d);
+    auto keys = [&](auto one, auto batch) {
+        if (ex.batch()) batch<<<blocks, 256, 0, st>>>(ex.args(kShapeCapN256L));
+        else one<<<blocks, 256, 0, st>>>(*ex.g, *ex.w);
+    };
+    switch (ex.d) {
+        case 2: keys(k_tile_keys<2>, kb_tile_keys<2>); break;
+        case 3: keys(k_tile_keys<3>, kb_tile_keys<3>); break;
+        case 4: keys(k_tile_keys<4>, kb_tile_keys<4>); break;
+        default: return;
+    }
+    for (int p = 0; p < P; p++) {
+        EGG_GO(ex, kShapeTiles, kSortThreads, st, tile_hist, p);
+        EGG_GO(ex, kShapeDigits, 256, st, tile_scan, p);
+        EGG_GO(ex, kShapeTiles, kSortThreads, st, tile_scatter, p);
+    }
 }
 
 void launch_cell_sums(const Exec& ex, cudaStream_t st) {

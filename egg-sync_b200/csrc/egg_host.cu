@@ -99,6 +99,8 @@ Geom make_geom(int64_t n64, int d, float eps) {
         g.zblk = g.width;
         g.nzb = 1;
     }
+    g.tile_min = kTileMinN;
+    g.point_walk = d > 4 || (d > 1 && !tile_capable(g));
     g.sub_dims = std::min(d, 8);
     g.sub_bits = std::max(1, 8 / g.sub_dims);
     return g;
@@ -163,13 +165,13 @@ size_t layout_work(const Geom& g, int max_iter, char* base, Work& w, float** xin
     add((void**)&w.smp, packed ? 16 * (size_t)pack_s(d) * ns : 0);
     add((void**)&w.qlo, 4 * d * ns);
     add((void**)&w.qhi, 4 * d * ns);
-    add((void**)&w.ulo, 4 * d * ns);
-    add((void**)&w.uhi, 4 * d * ns);
+    add((void**)&w.ubox, 4 * 2 * (size_t)box_w(d) * ns);
     add((void**)&w.orig, 4 * ns);
     add((void**)&w.orig_tmp, 4 * ns);
     add((void**)&w.perm, 4 * ns);
     add((void**)&w.perm_tmp, 4 * ns);
-    const bool one_key = d <= 3 && g.width <= 256;
+    // whole sort keys: of the grid sort (d <= 3, at most 256 cells per dimension) and of the tile order
+    const bool one_key = (d <= 3 && g.width <= 256) || tile_capable(g);
     add((void**)&w.skey[0], one_key ? 4 * ns : 0);
     add((void**)&w.skey[1], one_key ? 4 * ns : 0);
     if (!one_key) w.skey[0] = w.skey[1] = nullptr;  // the per-dimension passes
@@ -178,17 +180,18 @@ size_t layout_work(const Geom& g, int max_iter, char* base, Work& w, float** xin
     add((void**)&w.cell_dims, 4 * d * ns);
     add((void**)&w.cell_key, d <= 4 ? 8 * ns : 0);
     add((void**)&w.cell_outer, 4 * ns);
-    add((void**)&w.css, 4 * d * ns);
-    add((void**)&w.csm, 4 * d * ns);
-    add((void**)&w.cbmin, 4 * d * ns);
-    add((void**)&w.cbmax, 4 * d * ns);
+    const bool bytes = byte_keys(g);
+    add((void**)&w.cell_bytes, bytes ? 16 * ns : 0);
+    if (!bytes) w.cell_bytes = nullptr;
+    add((void**)&w.csum, 4 * (size_t)sum_w(d) * ns);
+    add((void**)&w.cbox, 4 * 2 * (size_t)box_w(d) * ns);
     add((void**)&w.outer_begin, 4 * ((size_t)g.n_outer + 1));
     add((void**)&w.colmask, g.od < d ? 8 * ((size_t)g.n_outer + 1) : 0);
     add((void**)&w.hist, 4 * 256 * (size_t)tiles);
     add((void**)&w.digit_total, 4 * 256);
     add((void**)&w.block_sums, 4 * (size_t)nb);
     add((void**)&w.wpart, 8 * 4 * (size_t)d * 2 * nw);
-    add((void**)&w.gpart, 4 * 4 * (size_t)d * 2 * nw);
+    add((void**)&w.gpart, 4 * (size_t)group_w(d) * 2 * nw);
     add((void**)&w.ctrl, 4 * kCtrlWords);
     add((void**)&w.ustats, 8 * kUStats);
     add((void**)&w.stamps, 8 * 4 * ((size_t)max_iter + 2));
@@ -409,7 +412,8 @@ __global__ void k_iter_end(Work w, cudaGraphConditionalHandle h, int in_graph, i
 // One iteration of the loop body.  With prof (8 events), the four kernel
 // groups are bracketed by CUDA events on the launching stream.
 // Parts of one iteration: 0 = begin + grid check, 1 = grid sort (skippable
-// when no point changed cell), 2 = the rest.  In the loop graph part 2 ends
+// when no point changed cell), 5 = the tile order of the new grid (skippable
+// where it does not pay), 2 = the rest.  In the loop graph part 2 ends
 // at the update (part 3 = the extra check, behind a conditional node; part 4
 // = the loop control).
 void enqueue_part(Instance& I, int part, cudaGraphConditionalHandle h, int in_graph, cudaEvent_t* prof = nullptr) {
@@ -425,6 +429,10 @@ void enqueue_part(Instance& I, int part, cudaGraphConditionalHandle h, int in_gr
     }
     if (part == 1) {
         launch_build_sort(single(I.g, I.w), st);
+        return;
+    }
+    if (part == 5) {
+        launch_tile_order(single(I.g, I.w), st);
         return;
     }
     if (part == 3) {
@@ -462,15 +470,20 @@ void enqueue_part(Instance& I, int part, cudaGraphConditionalHandle h, int in_gr
     k_iter_end<<<1, 1, 0, st>>>(I.w, h, in_graph, I.g.stop_rule);
 }
 
-// one iteration outside the loop graph (host-driven loop): parts 0-2, the
+// one iteration outside the loop graph (host-driven loop): parts 0, 1, 5, 2, the
 // last of which runs the extra check and the loop control itself
 void enqueue_iteration(Instance& I, cudaGraphConditionalHandle h, int in_graph, cudaEvent_t* prof = nullptr) {
-    for (int part = 0; part < 3; part++) enqueue_part(I, part, h, in_graph, prof);
+    for (int part : {0, 1, 5, 2}) enqueue_part(I, part, h, in_graph, prof);
 }
 
 // opens the grid-sort node of the loop graph when some point changed cell
 __global__ void k_gate_sort(Work w, cudaGraphConditionalHandle hs) {
     cudaGraphSetConditional(hs, w.ctrl[kCtrlChanged] != 0 ? 1u : 0u);
+}
+
+// ... and, after the sort, the tile-order node
+__global__ void k_gate_tile(Work w, cudaGraphConditionalHandle ht) {
+    cudaGraphSetConditional(ht, w.ctrl[kCtrlTileWant] != 0 ? 1u : 0u);
 }
 
 std::vector<char> graph_key(const Instance& I) {
@@ -523,13 +536,45 @@ bool ensure_graph(Instance& I) {
         cp.conditional.type = cudaGraphCondTypeIf;
         cp.conditional.size = 1;
         e = cudaGraphAddNode(&ifnode, body, &tail, 1, &cp);
+        // sort body: [sort, gate] -> IF(the new grid wants a tile order) [tile order]
+        const bool tile = tile_capable(I.g);
+        cudaGraph_t sbody = nullptr;
+        cudaGraphConditionalHandle ht;
+        cudaGraphNode_t stail = nullptr;
+        if (e == cudaSuccess) sbody = cp.conditional.phGraph_out[0];
+        if (e == cudaSuccess && tile) e = cudaGraphConditionalHandleCreate(&ht, sbody, 0, 0);
         if (e == cudaSuccess)
-            e = cudaStreamBeginCaptureToGraph(I.st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                              cudaStreamCaptureModeThreadLocal);
+            e = cudaStreamBeginCaptureToGraph(I.st, sbody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             enqueue_part(I, 1, h, 1);
+            if (tile) {
+                k_gate_tile<<<1, 1, 0, I.st>>>(I.w, ht);
+                cudaStreamCaptureStatus cs;
+                const cudaGraphNode_t* deps = nullptr;
+                size_t nd = 0;
+                e = cudaStreamGetCaptureInfo(I.st, &cs, nullptr, nullptr, &deps, &nd);
+                if (e == cudaSuccess && nd == 1) stail = deps[0];
+            }
             cudaGraph_t captured = nullptr;
-            e = cudaStreamEndCapture(I.st, &captured);
+            const cudaError_t e2 = cudaStreamEndCapture(I.st, &captured);
+            if (e == cudaSuccess) e = e2;
+            if (e == cudaSuccess && tile && !stail) e = cudaErrorUnknown;
+        }
+        if (e == cudaSuccess && tile) {
+            cudaGraphNodeParams tp = {cudaGraphNodeTypeConditional};
+            tp.conditional.handle = ht;
+            tp.conditional.type = cudaGraphCondTypeIf;
+            tp.conditional.size = 1;
+            cudaGraphNode_t tnode = nullptr;
+            e = cudaGraphAddNode(&tnode, sbody, &stail, 1, &tp);
+            if (e == cudaSuccess)
+                e = cudaStreamBeginCaptureToGraph(I.st, tp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                  cudaStreamCaptureModeThreadLocal);
+            if (e == cudaSuccess) {
+                enqueue_part(I, 5, h, 1);
+                cudaGraph_t captured = nullptr;
+                e = cudaStreamEndCapture(I.st, &captured);
+            }
         }
     }
     // ... -> [rest of the iteration up to the update, gate] -> IF(flag) [extra check] -> [loop control]
@@ -764,14 +809,18 @@ int run(const float* x, int64_t n, int32_t d, float eps, float lam, const egg_op
         const int sort_l = onekey ? 3 * (1 + g.d) + 5 : 3 * plan_count(g) + 4;
         const int build_l = sort_l + 2;
         const int order_l = (g.order_mode == 2 || g.stop_rule == 1) ? 2 : 0;
+        // tile order: keys and 3 kernels per pass; in the loop graph behind a
+        // gate of its own in every rebuild
+        const int tile_l = tile_capable(g) ? 1 + 3 * tile_passes(g.d) : 0;
         const int final_l = build_l + (opts.labels_mode == 1 ? 1 : 4) + (g.order_mode == 1 ? 4 : 0) +
                             (opts.positions_out ? 1 : 0);
-        long long loop_l = (long long)iters * (sort_l + 10 + order_l);
+        long long loop_l = (long long)iters * (sort_l + tile_l + 10 + order_l);
         if (use_graph) {
             // grid builds in the loop: all builds but the final one when it rebuilt
             const int loop_builds = I.h_ctrl[kCtrlBuilds] - (I.h_ctrl[kCtrlChanged] ? 1 : 0);
             loop_l = (long long)iters * (9 + order_l) + 3LL * I.h_ctrl[kCtrlExtraRuns] +
-                     (long long)loop_builds * sort_l;
+                     (long long)loop_builds * (sort_l + (tile_l ? 1 : 0)) +
+                     (long long)I.h_ctrl[kCtrlTileSorts] * tile_l;
         }
         stats->launches = (int32_t)(2 + loop_l + final_l + (opts.warm_start ? 10 : 0));
         stats->grid_builds = I.h_ctrl[kCtrlBuilds];
@@ -872,6 +921,7 @@ int step(const float* x, int64_t n, int32_t d, float eps, float* x_next, int32_t
     cudaStream_t st = I.st;
     k_iter_begin<<<1, 1, 0, st>>>(I.w);
     launch_build(single(I.g, I.w), st);
+    launch_tile_order(single(I.g, I.w), st);
     launch_cell_sums(single(I.g, I.w), st);
     launch_need(single(I.g, I.w), st);
     int* cnt_sorted = I.w.orig_tmp;  // free once the grid is built

@@ -25,8 +25,10 @@ struct BatchTables {
     int total[kShapeCount] = {};  // virtual blocks per shape over all instances
     int max_passes = 0;           // radix passes of the instance with the most
     int max_table_k = 0;
+    bool tile = false;            // some instance may want a tile order
+    bool bytes = false;           // every instance has byte keys (d > 4)
     int occ = 8;                  // persistent blocks per SM of a 256-thread kernel
-    int update_threads = 128;     // block size of the update kernel: 64, 128 or 256
+    int update_threads = 256;     // block size of the update kernel: 128 or 256
 };
 
 struct Exec {
@@ -34,6 +36,7 @@ struct Exec {
     const Work* w = nullptr;
     const BatchTables* bt = nullptr;   // batch
     int d = 0;                         // dimensions (kernel template)
+    bool tile = false;                 // some instance may want a tile order
     bool batch() const { return bt != nullptr; }
     // single: the shape's block count; batch: a persistent grid
     int blocks(int shape, int threads) const {
@@ -56,6 +59,7 @@ inline Exec single(const Geom& g, const Work& w) {
     e.g = &g;
     e.w = &w;
     e.d = g.d;
+    e.tile = tile_capable(g);
     return e;
 }
 
@@ -63,6 +67,7 @@ inline Exec batched(const BatchTables& bt, int d) {
     Exec e;
     e.bt = &bt;
     e.d = d;
+    e.tile = bt.tile;
     return e;
 }
 
@@ -74,6 +79,8 @@ void launch_build(const Exec& ex, cudaStream_t st);
 // begin = false: the caller's loop control already cleared the changed word.
 void launch_build_check(const Exec& ex, cudaStream_t st, bool begin = true);
 void launch_build_sort(const Exec& ex, cudaStream_t st);
+// the points of a rebuilt grid along a space-filling curve, for the update's warps
+void launch_tile_order(const Exec& ex, cudaStream_t st);
 void launch_cell_sums(const Exec& ex, cudaStream_t st);
 void launch_transpose_in(const Geom& g, const Work& w, const float* x, cudaStream_t st);
 void launch_unsort_positions(const Geom& g, const Work& w, const float* src, float* out, cudaStream_t st);
@@ -87,6 +94,8 @@ void launch_labels_uf(const Exec& ex, cudaStream_t st);
 // update + flag (egg_update.cu); counts (nullable, single instance only)
 // receives |N_eps(p)| per sorted point
 void launch_update(const Exec& ex, int* counts, cudaStream_t st);
+// d > 4 (egg_update_wide.cu)
+void launch_update_wide(const Exec& ex, int* counts, cudaStream_t st);
 // stencil dilation of the outer cells touched by moved points (incremental update)
 void launch_need(const Exec& ex, cudaStream_t st);
 
@@ -100,8 +109,9 @@ void launch_extra_check(const Exec& ex, cudaStream_t st, bool gated = false);
 void launch_gate_extra(const Work& w, cudaGraphConditionalHandle h, cudaStream_t st);
 // loop graph of a batch: the same per dimension group (any active instance flagged)
 void launch_batch_gate_extra(const Exec& ex, cudaGraphConditionalHandle h, cudaStream_t st);
-// ... and its grid sort (any active instance with a point that changed cell;
+// ... its tile order (any active instance that wants one), and its grid sort (any active instance with a point that changed cell;
 // *opened counts the openings)
+void launch_batch_gate_tile(const Exec& ex, cudaGraphConditionalHandle h, int* opened, cudaStream_t st);
 void launch_batch_gate_sort(const Exec& ex, cudaGraphConditionalHandle h, int* opened, cudaStream_t st);
 
 }  // namespace egg

@@ -41,7 +41,7 @@ __device__ __forceinline__ void order_cell(const Geom& g, const Work& w, int c, 
     if (!(sm2 <= g.t_eps)) return;
     const int qb = __ldg(w.cell_start + c), qe = __ldg(w.cell_start + c + 1);
     float near2, far2;
-    tight_box_dist2(x, w.cbmin + c, w.cbmax + c, g.ns, d, near2, far2);
+    tight_box_dist2<D>(x, cell_box<D>(w, c, d), d, near2, far2);
     const bool full = lg2 <= g.t_eps;
     if (!full && near2 > g.t_eps) return;
     if (full || far2 <= g.t_eps) {
@@ -50,19 +50,12 @@ __device__ __forceinline__ void order_cell(const Geom& g, const Work& w, int c, 
         return;
     }
     const int kh = qb >> 5, kt = (qe - 1) >> 5;
-    const int nw = (g.n + 31) >> 5;
     for (int k = kh; k <= kt; k++) {
         const int sb = max(qb, k << 5), se = min(qe, (k << 5) + 32);
         if (kh != kt) {
             const int rec = (k == kh) ? 1 : 0;
-            float n2 = 0.f, f2 = 0.f;
-            for (int l = 0; l < d; l++) {
-                const float L = __ldg(w.gpart + wp_idx_f(2, l, d, rec, nw, k));
-                const float H = __ldg(w.gpart + wp_idx_f(3, l, d, rec, nw, k));
-                const float a0 = near_gap(x[l], L, H), b0 = far_gap(x[l], L, H);
-                n2 = __fmaf_rn(a0, a0, n2);
-                f2 = __fmaf_rn(b0, b0, f2);
-            }
+            float n2, f2;
+            tight_box_dist2<D>(x, group_rec<D>(w, k, rec, d) + sum_w(d), d, n2, f2);
             if (n2 > g.t_eps) continue;
             if (f2 <= g.t_eps) {
                 add_interval(lo, hi, se - sb, n2, f2);
@@ -113,7 +106,7 @@ __global__ void __launch_bounds__(128) k_order_param(Geom g, Work w) {
         }
         double lo = 0.0, hi = 0.0;
         int N = 0;
-        for_candidates(g, w, gi, obase, lane, d, [] { return true; }, [&](int c) { order_cell<D>(g, w, c, x, lo, hi, N); });
+        for_candidates(g, w, gi, obase, lane, d, [] { return true; }, [](int) { return true; }, [&](int c) { order_cell<D>(g, w, c, x, lo, hi, N); });
         if (valid && N > 0) {
             rlo = lo / (double)N;
             rhi = hi / (double)N;

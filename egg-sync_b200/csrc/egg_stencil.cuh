@@ -16,7 +16,12 @@
 // Both paths give every lane the same results bit for bit: the extra cells
 // of the union fail that lane's box test.
 // fn(c) is called once per candidate cell per lane, in increasing stencil
-// entry then increasing cell order in both paths.  A lane for which
+// entry then increasing cell order in both paths.  col(s) is called before
+// the cells of stencil entry s (whole outer columns: every cell of one shares
+// its coordinates in the outer dimensions); a lane for which it returns false
+// needs no cell of that column.  Lockstep visits a column unless every lane
+// passes it over; a lane's own walk does not look the column up at all.
+// A lane for which
 // active() is false needs no result: it rides along in the lockstep path
 // and skips its own walk in the other (active() is evaluated there only, so
 // the lockstep path carries nothing extra).
@@ -42,19 +47,15 @@ __device__ __forceinline__ unsigned long long zwindow_mask(const Geom& g, int zl
     return (2ull << bh) - (1ull << bl);  // bits bl..bh (bh = 63 wraps to the right value)
 }
 
-template <typename A, typename F>
+template <typename A, typename C, typename F>
 __device__ __forceinline__ void for_candidates(const Geom& g, const Work& w, const int* gi, int obase, int lane,
-                                               int d, A&& active, F&& fn) {
+                                               int d, A&& active, C&& col, F&& fn) {
     const int nst = w.st_count[0];
     const int ob0 = __shfl_sync(0xffffffffu, obase, 0);
     int zlo = 0, zhi = 0;
     if (g.od < d) {
-        zlo = zhi = gi[g.od];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            zlo = min(zlo, __shfl_xor_sync(0xffffffffu, zlo, o));
-            zhi = max(zhi, __shfl_xor_sync(0xffffffffu, zhi, o));
-        }
+        zlo = __reduce_min_sync(0xffffffffu, gi[g.od]);
+        zhi = __reduce_max_sync(0xffffffffu, gi[g.od]);
     }
     if (__all_sync(0xffffffffu, obase == ob0) && zhi - zlo <= kLockZSpan) {
         for (int s0 = 0; s0 < nst; s0 += 32) {
@@ -83,6 +84,7 @@ __device__ __forceinline__ void for_candidates(const Geom& g, const Work& w, con
                 live &= live - 1;
                 const int b = __shfl_sync(0xffffffffu, cb, src);
                 const int e = __shfl_sync(0xffffffffu, ce, src);
+                if (!__any_sync(0xffffffffu, col(s0 + src))) continue;
                 for (int c = b; c < e; c++) fn(c);
             }
         }
@@ -113,7 +115,7 @@ __device__ __forceinline__ void for_candidates(const Geom& g, const Work& w, con
 #pragma unroll 1
             for (int k = 0; k < kAhead; k++) {
                 const int o = ol[k];
-                if (o < 0) continue;
+                if (o < 0 || !col(s0 + k)) continue;
                 int cb = __ldg(w.outer_begin + o), ce = __ldg(w.outer_begin + o + 1);
                 if (cb >= ce) continue;
                 if (g.od < d) {

@@ -19,8 +19,19 @@
 //
 // Cell classification, distance tests, the border rule and the flag follow
 // the reference exactly (EGG_SynC.cu:583-597, 613-636, 666-681, 706-709).
+//
+// d <= 4 (more dimensions: egg_update_wide.cu).  Bound by instruction issue
+// and by the latency of what is left of it, not by memory (the working set
+// stays in L2).  Grouping the update's threads along a space-filling curve
+// lets every warp walk in lockstep (before, 60% to 88% of the warps of the
+// first iterations had their lanes walk one by one): update kernel over the
+// first ten iterations, 1M x 3D 60 -> 40 ms, 250k x 3D 23.0 -> 15.0,
+// 45,781 x 3D 9.5 -> 4.7, 100k x 4D 17.9 -> 8.2 ms, all bit-identical.
+#include <climits>
+
 #include "egg_common.cuh"
 #include "egg_kernels.h"
+#include "egg_point_walk.cuh"
 #include "egg_stencil.cuh"
 
 namespace egg {
@@ -32,8 +43,7 @@ namespace {
 // within eps/2 in the other fully covered cells.
 template <int D>
 __device__ int half_count(const Geom& g, const Work& w, const float* x, const int* gi, int obase, int own, int own_cnt) {
-    constexpr int DM = D > 0 ? D : kMaxDims;
-    const int d = D > 0 ? D : g.d;
+    constexpr int d = D;
     int half = own_cnt;
     const int nst = w.st_count[0];
     for (int s = 0; s < nst; s++) {
@@ -58,7 +68,7 @@ __device__ int half_count(const Geom& g, const Work& w, const float* x, const in
             if (!(lg2 <= g.t_eps)) continue;
             const int qb = __ldg(w.cell_start + c), qe = __ldg(w.cell_start + c + 1);
             float near2, far2;
-            tight_box_dist2(x, w.cbmin + c, w.cbmax + c, g.ns, d, near2, far2);
+            tight_box_dist2<D>(x, cell_box<D>(w, c, d), d, near2, far2);
             if (near2 > g.t_half) continue;
             if (far2 <= g.t_half) {
                 half += qe - qb;
@@ -71,7 +81,6 @@ __device__ int half_count(const Geom& g, const Work& w, const float* x, const in
             }
         }
     }
-    (void)DM;
     return half;
 }
 
@@ -85,13 +94,34 @@ namespace {
 #define EGG_STAT(a, k, v) ((void)0)
 #endif
 
+// The outer column a walk is in: the box terms and cell offsets of the outer
+// dimensions (l < od) are the same for every cell of the column, so they are
+// formed once per column and point.  The box sums start with the outer
+// dimensions, in the same order, so the totals round alike.
+template <int D>
+struct Col {
+    float sm, lg;
+    int kk[D];
+};
+
+// Lockstep walks read points from shared memory four at a time:
+// with two in flight the loop waits on each load (1M x 3D: 42 -> 47 ms for
+// the first ten iterations).  They want registers more than warps: five
+// blocks of 128 threads per SM (96 registers) beat four (47 ms), six (80
+// registers, 47 ms) and eight (64 registers, 45 ms); d = 4 keeps four blocks
+// (100k x 4D: 12.4 ms against 13.5).
+constexpr int kWalkUnroll = 4;
+constexpr int update_min_blocks(int d, int threads) {
+    const int m = (d <= 3 ? 640 : 512) / threads;
+    return m > 0 ? m : 1;
+}
+
 template <int D>
 struct Acc {
-    float S[D > 0 ? D : kMaxDims];
-    float Cm[D > 0 ? D : kMaxDims];
+    float S[D];
+    float Cm[D];
     int N;
     int partial_in;
-    bool tab_err;
 #ifdef EGG_UPDATE_STATS
     unsigned st[kUStats];
 #endif
@@ -99,411 +129,652 @@ struct Acc {
 
 // m counted points of a cell at offsets k (= cell dims - own dims) with
 // SS = sum sin(delta), SM = sum (1 - cos(delta)) into the own-cell frame.
+// tab[k + K] = sin(k side), cos(k side), 1 - cos(k side): one 16-byte load.
 template <int D>
-__device__ __forceinline__ void add_counted(Acc<D>& a, int d, const int* kk, float m, const float* SS, const float* SM,
-                                            const float* Ts, const float* Tc, const float* Tm, int K, int TW) {
-    for (int l = 0; l < d; l++) {
-        int k = kk[l] + K;
-        if ((unsigned)k >= (unsigned)TW) { a.tab_err = true; k = K; }
-        const float ts = Ts[k], tc = Tc[k], tm = Tm[k];
+__device__ __forceinline__ void add_counted(Acc<D>& a, const int* kk, float m, const float* SS, const float* SM,
+                                            const float4* tab, int K) {
+#pragma unroll
+    for (int l = 0; l < D; l++) {
+        const float4 t = tab[kk[l] + K];
+        const float ts = t.x, tc = t.y, tm = t.z;
         a.S[l] += ts * (m - SM[l]) + tc * SS[l];
         a.Cm[l] += m * tm + tc * SM[l] + ts * SS[l];
     }
 }
 
-// One candidate cell for one point: the reference's box test
-// (EGG_SynC.cu:613-636), then the aggregate (fully covered, or all points
-// provably within eps), nothing (no point provably within eps), or a walk.
+// cell coordinate l from the packed 16-bit key, as a float without the
+// integer-to-float unit: the 16 bits are the low mantissa of 2^23 + cd
+__device__ __forceinline__ float key_dim_f(unsigned long long key, int l) {
+    const unsigned word = (unsigned)(key >> (32 * (l >> 1)));
+    const unsigned bits = __byte_perm(word, 0x4b000000u, (l & 1) ? 0x7432 : 0x7410);
+    return __uint_as_float(bits) - 8388608.0f;
+}
+// box_terms with the cell coordinate as a float: the smaller square to sm,
+// the larger to lg (equal squares are the same addend either way)
+__device__ __forceinline__ void box_terms_f(float x, float cd, float side, float& sm, float& lg) {
+    const float left = __fmaf_rn(cd, side, -x);
+    const float right = __fmaf_rn(cd + 1.0f, side, -x);
+    const float l2 = __fmul_rn(left, left), r2 = __fmul_rn(right, right);
+    sm = __fadd_rn(sm, fminf(l2, r2));
+    lg = __fadd_rn(lg, fmaxf(l2, r2));
+}
+
+// two floats of a register pair, added or subtracted in one instruction
+// (each half rounds to nearest as the scalar operation does)
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// squared distance to a packed point, the operations and order of dist_step;
+// nx holds -x in pairs
 template <int D>
-__device__ __forceinline__ void visit_cell(const Geom& g, const Work& w, int c, const float* x, const int* gi,
-                                           Acc<D>& a, const float* Ts, const float* Tc, const float* Tm, int K, int TW) {
-    constexpr int DM = D > 0 ? D : kMaxDims;
-    const int d = D > 0 ? D : g.d;
-    float sm2 = 0.f, lg2 = 0.f;
-    int kk[DM];
-    if constexpr (D >= 1 && D <= 4) {
-        // the cell's dims from one packed word
-        const unsigned long long key = __ldg(w.cell_key + c);
+__device__ __forceinline__ float pair_dist2(const ulonglong2* v, const unsigned long long* nx, const float* x) {
+    float acc = 0.f;
 #pragma unroll
-        for (int l = 0; l < D; l++) {
-            const int cd = (int)((key >> (16 * l)) & 0xffffu);
-            box_terms(x[l], cd, g.side, sm2, lg2);
-            kk[l] = cd - gi[l];
+    for (int j = 0; j < pack_w(D); j++) {
+        float e0, e1, e2 = 0.f, e3 = 0.f;
+        unpack2(add2(v[j].x, nx[2 * j]), e0, e1);
+        if (4 * j + 3 < D) {
+            unpack2(add2(v[j].y, nx[2 * j + 1]), e2, e3);
+        } else if (4 * j + 2 < D) {
+            unpack2(v[j].y, e2, e3);
+            e2 = __fsub_rn(e2, x[4 * j + 2 < D ? 4 * j + 2 : 0]);
         }
-    } else {
-        for (int l = 0; l < d; l++) {
-            const int cd = __ldg(w.cell_dims + (size_t)l * g.ns + c);
-            box_terms(x[l], cd, g.side, sm2, lg2);
-            kk[l] = cd - gi[l];
-        }
+        acc = __fmaf_rn(e0, e0, acc);
+        if (4 * j + 1 < D) acc = __fmaf_rn(e1, e1, acc);
+        if (4 * j + 2 < D) acc = __fmaf_rn(e2, e2, acc);
+        if (4 * j + 3 < D) acc = __fmaf_rn(e3, e3, acc);
     }
+    return acc;
+}
+
+// tight_box_dist2 on a box record (lower, then upper corner) read in whole
+// words, the differences of two dimensions at a time: lo - x and hi - x give
+// the near gap max(lo - x, x - hi, 0) and the far gap max(|lo - x|, |hi - x|)
+template <int D, bool kGlobal>
+__device__ __forceinline__ void box_dist2(const unsigned long long* nx, const float* x, const ulonglong2* box,
+                                          float& near2, float& far2) {
+    float a2 = 0.f, b2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < pack_w(D); j++) {
+        const ulonglong2 L = kGlobal ? __ldg(box + j) : box[j];
+        const ulonglong2 H = kGlobal ? __ldg(box + pack_w(D) + j) : box[pack_w(D) + j];
+        float dl[4], dh[4];
+        unpack2(add2(L.x, nx[2 * j]), dl[0], dl[1]);
+        unpack2(add2(H.x, nx[2 * j]), dh[0], dh[1]);
+        if (4 * j + 3 < D) {
+            unpack2(add2(L.y, nx[2 * j + 1]), dl[2], dl[3]);
+            unpack2(add2(H.y, nx[2 * j + 1]), dh[2], dh[3]);
+        } else if (4 * j + 2 < D) {
+            unpack2(L.y, dl[2], dl[3]);
+            unpack2(H.y, dh[2], dh[3]);
+            dl[2] = __fsub_rn(dl[2], x[4 * j + 2 < D ? 4 * j + 2 : 0]);
+            dh[2] = __fsub_rn(dh[2], x[4 * j + 2 < D ? 4 * j + 2 : 0]);
+        }
+#pragma unroll
+        for (int l = 0; l < 4; l++)
+            if (4 * j + l < D) {
+                const float near = fmaxf(fmaxf(dl[l], -dh[l]), 0.f), far = fmaxf(fabsf(dl[l]), fabsf(dh[l]));
+                a2 = __fmaf_rn(near, near, a2);
+                b2 = __fmaf_rn(far, far, b2);
+            }
+    }
+    near2 = a2;
+    far2 = b2;
+}
+
+// a sum record (a point's, a group's) added to the pairs av
+template <int D, bool kGlobal>
+__device__ __forceinline__ void add_point(unsigned long long* av, const ulonglong2* rec) {
+#pragma unroll
+    for (int j = 0; j < pack_s(D); j++) {
+        const ulonglong2 t = kGlobal ? __ldg(rec + j) : rec[j];
+        av[2 * j] = add2(av[2 * j], t.x);
+        if (4 * j + 2 < 2 * D) av[2 * j + 1] = add2(av[2 * j + 1], t.y);
+    }
+}
+
+// -x in pairs
+template <int D>
+__device__ __forceinline__ void negate_pairs(const float* x, unsigned long long* nx) {
+#pragma unroll
+    for (int k = 0; k < 2 * pack_w(D); k++)
+        nx[k] = pack2(2 * k < D ? -x[2 * k < D ? 2 * k : 0] : 0.f, 2 * k + 1 < D ? -x[2 * k + 1 < D ? 2 * k + 1 : 0] : 0.f);
+}
+
+// ---------------------------------------------------------------------------
+// The walk of a whole warp in lockstep (d <= 4).
+//
+// The warp takes the columns within r of any active lane's cell, each
+// restricted in dimension od to the lanes' joint window.  Columns ascend and a
+// column's cells ascend, so every lane meets its own candidates in the order
+// of its own stencil; cells beyond its stencil it passes over (in the outer
+// dimensions by their offset, elsewhere they fail its box test).  The
+// candidates come 32 at a time, one per lane: each lane reads its cell's
+// record, drops it when no active lane can count any of its points, and
+// leaves it in shared memory otherwise.  Then the warp goes through the kept
+// cells one by one, reading the records as broadcasts: no visit waits for a
+// chain of loads, and the cells that only widen the joint window (40% of
+// them) cost a thirty-second of a visit.
+//
+// With the joint box too wide the walk does not pay and returns false before
+// any visit: in storage order (tiled false) as soon as the lanes lie in
+// several columns or spread over dimension od (consecutive points of sparse
+// columns are dozens of cells apart there), in tile order only for more than
+// kUnionCols columns (points of an empty region).
+// ---------------------------------------------------------------------------
+constexpr int kUnionCols = 1024;
+
+// shared memory of one warp, in 16-byte words: its joint box, 32 cell records (key, first
+// point, points | box | sums), then 32 points (coordinates | sums)
+__host__ __device__ constexpr int cell_words(int d) { return 1 + 2 * pack_w(d) + pack_s(d); }
+__host__ __device__ constexpr int box_words(int d) { return (4 * (5 * d + 2) + 15) / 16; }
+__host__ __device__ constexpr int warp_words(int d) { return box_words(d) + 32 * cell_words(d) + 32 * (pack_w(d) + pack_s(d)); }
+
+// float order as unsigned order, and back
+__device__ __forceinline__ unsigned order_key(float x) {
+    const unsigned u = __float_as_uint(x);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float order_val(unsigned k) {
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+// One kept cell for the 32 lanes; a lane whose column is off (col.sm infinite)
+// contributes nothing.  A group of points that some lane has to walk is
+// brought into shared memory by the whole warp (one coalesced load per record
+// word instead of a dependent load per point), then every walking lane reads
+// the points as broadcasts.
+template <int D, int OD>
+__device__ __forceinline__ void visit_cell_warp(const Geom& g, const Work& w, const ulonglong2* rec, const float* x,
+                                                const unsigned long long* nx, const int* gi, const Col<D>& col,
+                                                Acc<D>& a, const float4* tab, int K, ulonglong2* stage, int lane) {
+    constexpr int PW = pack_w(D), PS = pack_s(D);
+    const int od = OD > 0 ? OD : g.od;
+    const ulonglong2 head = rec[0];
+    const unsigned long long key = head.x;
+    float sm2 = col.sm, lg2 = col.lg;
+#pragma unroll
+    for (int l = 0; l < D; l++)
+        if (l >= od) box_terms_f(x[l], key_dim_f(key, l), g.side, sm2, lg2);
+    const bool pass = sm2 <= g.t_eps;
     EGG_STAT(a, kUsCells, 1);
-    if (!(sm2 <= g.t_eps)) return;
-    EGG_STAT(a, kUsSmallPass, 1);
-    const int qb = __ldg(w.cell_start + c), qe = __ldg(w.cell_start + c + 1);
-    bool all_in = lg2 <= g.t_eps;
-    const bool full = all_in;
-    if (!full) {
-        float near2, far2;
-        tight_box_dist2(x, w.cbmin + c, w.cbmax + c, g.ns, d, near2, far2);
-        if (near2 > g.t_eps) {
-            EGG_STAT(a, kUsTightOut, 1);
-            return;
-        }
-        all_in = far2 <= g.t_eps;
-        if (all_in) EGG_STAT(a, kUsTightIn, 1);
-    } else {
-        EGG_STAT(a, kUsFull, 1);
-    }
-    if (all_in) {
-        float SS[DM], SM[DM];
-        for (int l = 0; l < d; l++) {
-            SS[l] = __ldg(w.css + (size_t)l * g.ns + c);
-            SM[l] = __ldg(w.csm + (size_t)l * g.ns + c);
-        }
-        add_counted<D>(a, d, kk, (float)(qe - qb), SS, SM, Ts, Tc, Tm, K, TW);
-        a.N += qe - qb;
-        if (!full) a.partial_in += qe - qb;
-        return;
-    }
-    float as[DM], am[DM];
-    for (int l = 0; l < d; l++) { as[l] = 0.f; am[l] = 0.f; }
+    if (!__any_sync(0xffffffffu, pass)) return;
+    const int qb = (int)(unsigned)head.y, m_all = (int)(unsigned)(head.y >> 32);
+    float near2, far2;
+    box_dist2<D, false>(nx, x, rec + 1, near2, far2);
+    const bool full = lg2 <= g.t_eps;
+    const bool in = pass && (full || far2 <= g.t_eps);
+    const bool straddle = pass && !in && !(near2 > g.t_eps);
+    EGG_STAT(a, kUsSmallPass, pass);
+    EGG_STAT(a, kUsFull, pass && full);
+    EGG_STAT(a, kUsTightIn, in && !full);
+    EGG_STAT(a, kUsTightOut, pass && !in && !straddle);
+    if (!__any_sync(0xffffffffu, in || straddle)) return;
+    // counted points and their sums: the whole cell's, or the walked ones
+    unsigned long long av[2 * PS];
     int cnt = 0;
-    const int kh = qb >> 5, kt = (qe - 1) >> 5;
-    for (int k = kh; k <= kt; k++) {
-        // the cell's points in warp k: one 32-point group of a cell ordered
-        // along the sub-cell curve; its tight box decides it wholesale when
-        // all or none of its points are within eps
-        const int sb = max(qb, k << 5), se = min(qe, (k << 5) + 32);
-        if (kh != kt) {
-            const int nw = (g.n + 31) >> 5;
-            const int rec = (k == kh) ? 1 : 0;
-            float n2 = 0.f, f2 = 0.f;
-            for (int l = 0; l < d; l++) {
-                const float L = __ldg(w.gpart + wp_idx_f(2, l, d, rec, nw, k));
-                const float H = __ldg(w.gpart + wp_idx_f(3, l, d, rec, nw, k));
-                const float a0 = near_gap(x[l], L, H), b0 = far_gap(x[l], L, H);
-                n2 = __fmaf_rn(a0, a0, n2);
-                f2 = __fmaf_rn(b0, b0, f2);
-            }
-            if (n2 > g.t_eps) {
-                EGG_STAT(a, kUsGroupsOut, 1);
-                continue;
-            }
-            if (f2 <= g.t_eps) {
-                EGG_STAT(a, kUsGroupsIn, 1);
-                for (int l = 0; l < d; l++) {
-                    as[l] += __ldg(w.gpart + wp_idx_f(0, l, d, rec, nw, k));
-                    am[l] += __ldg(w.gpart + wp_idx_f(1, l, d, rec, nw, k));
-                }
-                cnt += se - sb;
-                continue;
-            }
+#pragma unroll
+    for (int k = 0; k < 2 * PS; k++) av[k] = 0ull;
+    if (in) {
+#pragma unroll
+        for (int j = 0; j < PS; j++) {
+            const ulonglong2 t = rec[1 + 2 * PW + j];
+            av[2 * j] = t.x;
+            av[2 * j + 1] = t.y;
         }
-        EGG_STAT(a, kUsPairs, se - sb);
-        if constexpr (D >= 1 && D <= kPackDims) {
-            // packed records: one or two 16-byte loads per candidate point
-            constexpr int PW = pack_w(D > 0 ? D : 1), PS = pack_s(D > 0 ? D : 1);
-            const float4* xp = w.xp + (size_t)sb * PW;
-            const float4* sp = w.smp + (size_t)sb * PS;
-            for (int q = sb; q < se; q++, xp += PW, sp += PS) {
+        cnt = m_all;
+    }
+    if (__any_sync(0xffffffffu, straddle)) {
+        const int qe = qb + m_all;
+        const int kh = qb >> 5, kt = (qe - 1) >> 5;
+        for (int k = kh; k <= kt; k++) {
+            const int sb = max(qb, k << 5), se = min(qe, (k << 5) + 32);
+            const int m = se - sb;
+            bool walk = straddle;
+            if (kh != kt) {
+                const ulonglong2* gr = reinterpret_cast<const ulonglong2*>(group_rec<D>(w, k, (k == kh) ? 1 : 0, D));
+                float n2, f2;
+                box_dist2<D, true>(nx, x, gr + PS, n2, f2);
+                const bool g_in = straddle && !(n2 > g.t_eps) && f2 <= g.t_eps;
+                walk = straddle && !(n2 > g.t_eps) && !g_in;
+                EGG_STAT(a, kUsGroupsOut, straddle && n2 > g.t_eps);
+                EGG_STAT(a, kUsGroupsIn, g_in);
+                if (g_in) {
+                    add_point<D, true>(av, gr);
+                    cnt += m;
+                }
+            }
+            if (!__any_sync(0xffffffffu, walk)) continue;
+            __syncwarp();
+            if (lane < m) {
+                const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(w.xp) + (size_t)(sb + lane) * PW;
+#pragma unroll
+                for (int j = 0; j < PW; j++) stage[lane * PW + j] = __ldg(xp + j);
+                const ulonglong2* sp = reinterpret_cast<const ulonglong2*>(w.smp) + (size_t)(sb + lane) * PS;
+#pragma unroll
+                for (int j = 0; j < PS; j++) stage[32 * PW + lane * PS + j] = __ldg(sp + j);
+            }
+            __syncwarp();
+            if (walk) {
+                EGG_STAT(a, kUsPairs, m);
+#pragma unroll kWalkUnroll
+                for (int j = 0; j < m; j++) {
 #ifdef EGG_UPDATE_STATS
-                {
-                    const unsigned am_ = __activemask();
-                    if ((threadIdx.x & 31) == __ffs(am_) - 1) a.st[kUsWalkSteps] += 1;
-                }
+                    {
+                        const unsigned am_ = __activemask();
+                        if ((threadIdx.x & 31) == __ffs(am_) - 1) a.st[kUsWalkSteps] += 1;
+                    }
 #endif
-                float xq[4 * PW];
-#pragma unroll
-                for (int k = 0; k < PW; k++) {
-                    const float4 v = __ldg(xp + k);
-                    xq[4 * k] = v.x;
-                    xq[4 * k + 1] = v.y;
-                    xq[4 * k + 2] = v.z;
-                    xq[4 * k + 3] = v.w;
-                }
-                float d2 = 0.f;
-#pragma unroll
-                for (int l = 0; l < DM; l++) d2 = dist_step(xq[l], x[l], d2);
-                if (d2 <= g.t_eps) {
-                    float v[4 * PS];
-#pragma unroll
-                    for (int k = 0; k < PS; k++) {
-                        const float4 t = __ldg(sp + k);
-                        v[4 * k] = t.x;
-                        v[4 * k + 1] = t.y;
-                        v[4 * k + 2] = t.z;
-                        v[4 * k + 3] = t.w;
+                    if (pair_dist2<D>(stage + j * PW, nx, x) <= g.t_eps) {
+                        add_point<D, false>(av, stage + 32 * PW + j * PS);
+                        cnt++;
                     }
-#pragma unroll
-                    for (int l = 0; l < DM; l++) {
-                        as[l] += v[l];
-                        am[l] += v[DM + l];
-                    }
-                    cnt++;
-                }
-            }
-        } else {
-            for (int q = sb; q < se; q++) {
-                float d2 = 0.f;
-                for (int l = 0; l < d; l++) d2 = dist_step(__ldg(w.X + (size_t)l * g.ns + q), x[l], d2);
-                if (d2 <= g.t_eps) {
-                    for (int l = 0; l < d; l++) {
-                        as[l] += __ldg(w.sd + (size_t)l * g.ns + q);
-                        am[l] += __ldg(w.md + (size_t)l * g.ns + q);
-                    }
-                    cnt++;
                 }
             }
         }
+        EGG_STAT(a, kUsPairsIn, in ? 0 : cnt);
     }
     if (cnt) {
-        add_counted<D>(a, d, kk, (float)cnt, as, am, Ts, Tc, Tm, K, TW);
+        float v[4 * PS];
+        int kk[D];
+#pragma unroll
+        for (int j = 0; j < 2 * PS; j++) unpack2(av[j], v[2 * j], v[2 * j + 1]);
+#pragma unroll
+        for (int l = 0; l < D; l++) kk[l] = l < od ? col.kk[l] : (int)((key >> (16 * l)) & 0xffffu) - gi[l];
+        // every offset is within the table: the lane passed the cell's box test
+        add_counted<D>(a, kk, (float)cnt, v, v + D, tab, K);
         a.N += cnt;
-        a.partial_in += cnt;
+        if (!full) a.partial_in += cnt;
     }
-    EGG_STAT(a, kUsPairsIn, cnt);
+}
+
+// what the screening of candidates needs of the warp's joint box: the same for
+// all lanes, so it waits in shared memory (volatile: read where it is used)
+// instead of in every lane's registers
+template <int D>
+struct WarpBox {
+    int lo[D], hi[D], wide[D];
+    float xl[D], xh[D];
+    float mar, r2;
+};
+
+template <int D, int OD>
+__device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const float* x, const int* gi, bool act,
+                                           bool tiled, Acc<D>& a, const float4* tab, int K, ulonglong2* sh,
+                                           int lane) {
+    constexpr int PW = pack_w(D), PS = pack_s(D), CW = cell_words(D);
+    const int od = OD > 0 ? OD : g.od;
+    static_assert(sizeof(WarpBox<D>) <= 16 * box_words(D), "the joint box's words");
+    volatile WarpBox<D>& B = *reinterpret_cast<WarpBox<D>*>(sh);
+    ulonglong2* const cells = sh + box_words(D);
+    ulonglong2* const stage = cells + 32 * CW;
+    int ncol;
+    {
+        float cols = 1.f, mar = 1.f;
+        bool one = true;
+#pragma unroll
+        for (int l = 0; l < D; l++) {
+            const int lo = __reduce_min_sync(0xffffffffu, act ? gi[l] : INT_MAX);
+            const int hi = __reduce_max_sync(0xffffffffu, act ? gi[l] : INT_MIN);
+            const int wide = l < od ? min(g.width - 1, hi + g.r) - max(0, lo - g.r) + 1 : 1;
+            cols *= (float)wide;
+            if (l < od) one = one && lo == hi;
+            if (l == od) one = one && hi - lo <= kLockZSpan;
+            // the active lanes' bounding box, and a margin for the rounding of
+            // the faces' offsets (relative to the coordinates)
+            const float xl = order_val(__reduce_min_sync(0xffffffffu, act ? order_key(x[l]) : 0xffffffffu));
+            const float xh = order_val(__reduce_max_sync(0xffffffffu, act ? order_key(x[l]) : 0u));
+            mar = fmaxf(mar, fmaxf(fabsf(xl), fabsf(xh)));
+            if (lane == 0) {
+                B.lo[l] = lo;
+                B.hi[l] = hi;
+                B.wide[l] = wide;
+                B.xl[l] = xl;
+                B.xh[l] = xh;
+            }
+        }
+        if (tiled ? cols > (float)kUnionCols : !one) return false;
+        ncol = (int)cols;
+        if (lane == 0) {
+            const float inv = 1.0f / g.side;
+            B.mar = mar * 4e-7f;
+            B.r2 = g.t_eps * inv * inv * 1.002f;
+        }
+        __syncwarp();
+    }
+    unsigned long long nx[2 * PW];
+    negate_pairs<D>(x, nx);
+    Col<D> col;
+    col.sm = col.lg = 0.f;
+    const int ob = 16 * od;
+    const unsigned long long outer = ob >= 64 ? ~0ull : (1ull << ob) - 1ull;  // a packed key's outer coordinates
+    for (int s0 = 0; s0 < ncol; s0 += 32) {
+        // a column per lane: its candidate cells [cb, ce)
+        int cb = 0, ce = 0;
+        {
+            int rem = s0 + lane, o = 0;
+            float exc = rem < ncol ? 0.f : INFINITY;
+#pragma unroll
+            for (int l = 0; l < D; l++)
+                if (l < od) {
+                    const int wide = B.wide[l], lo = B.lo[l];
+                    const int q = rem / wide;
+                    const int v = max(0, lo - g.r) + rem - q * wide;
+                    rem = q;
+                    o += v * g.wpow[l];
+                    // no lane's cell is nearer than this many cells
+                    const float gap = (float)max(max(lo - v, v - B.hi[l]), 0) - 1.001f;
+                    exc += gap > 0.f ? gap * gap : 0.f;
+                }
+            if (exc <= B.r2) {
+                cb = __ldg(w.outer_begin + o);
+                ce = __ldg(w.outer_begin + o + 1);
+                if (cb < ce && od < D) {
+                    const int* keys = w.cell_dims + (size_t)od * g.ns;
+                    cb = lower_bound_i(keys, cb, ce, B.lo[od < D ? od : 0] - g.r - 1);
+                    ce = lower_bound_i(keys, cb, ce, B.hi[od < D ? od : 0] + g.r + 2);
+                }
+            }
+        }
+        // the chunk's candidates numbered through, column by column
+        int upto = ce - cb;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, upto, k);
+            if (lane >= k) upto += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, upto, 31);
+        const int shift = ce - upto;  // candidate f of this column is cell f + shift
+        for (int f0 = 0; f0 < total; f0 += 32) {
+            const int f = f0 + lane;
+            bool keep = f < total;
+            int nk;
+            {
+                // the column holding candidate f: the first with upto > f
+                int src = 0;
+#pragma unroll
+                for (int k = 16; k > 0; k >>= 1) {
+                    const int t = __shfl_sync(0xffffffffu, upto, src + k - 1);
+                    if (t <= f) src += k;
+                }
+                src = min(src, 31);
+                const int c = f + __shfl_sync(0xffffffffu, shift, src);
+                unsigned long long key = 0;
+                ulonglong2 bl[2 * PW];
+                int qb = 0, qe = 0;
+                if (keep) {
+                    key = __ldg(w.cell_key + c);
+                    qb = __ldg(w.cell_start + c);
+                    qe = __ldg(w.cell_start + c + 1);
+                    const ulonglong2* bp = reinterpret_cast<const ulonglong2*>(cell_box<D>(w, c, D));
+#pragma unroll
+                    for (int j = 0; j < 2 * PW; j++) bl[j] = __ldg(bp + j);
+                    // no active lane passes the cell's box test, or no point of
+                    // it is within eps of any (the tight box; a cell at the
+                    // grid's edge also holds points beyond its own box and may
+                    // count in full all the same)
+                    float L[4 * PW], H[4 * PW], box2 = 0.f, tight2 = 0.f;
+#pragma unroll
+                    for (int j = 0; j < PW; j++) {
+                        unpack2(bl[j].x, L[4 * j], L[4 * j + 1]);
+                        unpack2(bl[j].y, L[4 * j + 2], L[4 * j + 3]);
+                        unpack2(bl[PW + j].x, H[4 * j], H[4 * j + 1]);
+                        unpack2(bl[PW + j].y, H[4 * j + 2], H[4 * j + 3]);
+                    }
+                    bool edge = false;
+                    const float mar = B.mar, t_out = g.t_eps * 1.0001f;
+#pragma unroll
+                    for (int l = 0; l < D; l++) {
+                        const float cd = key_dim_f(key, l), xl = B.xl[l], xh = B.xh[l];
+                        const float gb = fmaxf(fmaxf(cd * g.side - xh, xl - (cd + 1.0f) * g.side) - mar, 0.f);
+                        const float gt = fmaxf(fmaxf(L[l] - xh, xl - H[l]) - mar, 0.f);
+                        box2 = fmaf(gb, gb, box2);
+                        tight2 = fmaf(gt, gt, tight2);
+                        edge = edge || cd == 0.f || cd >= (float)(g.width - 1);
+                    }
+                    keep = !(box2 > t_out) && (edge || !(tight2 > t_out));
+                }
+                const unsigned kept = __ballot_sync(0xffffffffu, keep);
+                nk = __popc(kept);
+                __syncwarp();  // the last chunk's records are read
+                if (keep) {
+                    ulonglong2* rec = cells + __popc(kept & ((1u << lane) - 1u)) * CW;
+                    const ulonglong2* sp = reinterpret_cast<const ulonglong2*>(cell_sum<D>(w, c, D));
+                    rec[0] = make_ulonglong2(key, (unsigned long long)(unsigned)qb |
+                                                      ((unsigned long long)(unsigned)(qe - qb) << 32));
+#pragma unroll
+                    for (int j = 0; j < 2 * PW; j++) rec[1 + j] = bl[j];
+#pragma unroll
+                    for (int j = 0; j < PS; j++) rec[1 + 2 * PW + j] = __ldg(sp + j);
+                }
+                __syncwarp();
+            }
+            unsigned long long at = ~0ull;  // outer coordinates of the column col describes
+#pragma unroll 1
+            for (int j = 0; j < nk; j++) {
+                const ulonglong2* rec = cells + j * CW;
+#ifdef EGG_UPDATE_STATS
+                const long long tv = clock64();
+#endif
+                const unsigned long long ck = rec[0].x & outer;
+                if (ck != at) {
+                    at = ck;
+                    float sm = 0.f, lg = 0.f;
+                    bool on = act;
+#pragma unroll
+                    for (int l = 0; l < D; l++)
+                        if (l < od) {
+                            const int k = (int)((ck >> (16 * l)) & 0xffffu) - gi[l];
+                            col.kk[l] = k;
+                            on = on && abs(k) <= g.r;
+                            box_terms_f(x[l], key_dim_f(ck, l), g.side, sm, lg);
+                        }
+                    col.sm = on ? sm : INFINITY;
+                    col.lg = lg;
+                }
+                visit_cell_warp<D, OD>(g, w, rec, x, nx, gi, col, a, tab, K, stage, lane);
+#ifdef EGG_UPDATE_STATS
+                if (lane == 0) {
+                    a.st[kUsWarpVisits] += 1;
+                    a.st[kUsCyclesVisits] += (unsigned)(clock64() - tv);
+                }
+#endif
+            }
+        }
+    }
+    return true;
 }
 
 }  // namespace
 
-// One thread per cell-sorted point.  When the 32 points of a warp share one
-// outer cell (the common case: sorted points are grouped by outer cell), the
-// warp resolves the stencil's outer cells in parallel (lane = stencil entry)
-// and then visits every candidate cell with all lanes in lockstep, so cell
-// records are broadcast loads and the dependent-load chain of the stencil
-// walk is paid once per warp instead of once per point.  Otherwise each lane
-// walks the stencil on its own.  Both paths visit a superset of the cells
-// the reference visits and apply the reference's per-point box test to each.
-template <int D>
-__device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* __restrict__ counts, int bx) {
-    constexpr int DM = D > 0 ? D : kMaxDims;
-    const int d = D > 0 ? D : g.d;
-    extern __shared__ float s_tab[];
+// One thread per point.  In tile order a warp's points are neighbours in
+// space; otherwise they are 32 in a row of the storage order, the block's
+// warps taking rows from all over it (the points that still move late in a
+// run sit together, and a block shares them out).  A warp none of whose
+// points is touched keeps them all; one whose points are close enough walks
+// their joint candidates in lockstep; the points of any other go on the
+// block's list, and its warps take them one at a time (walk_point).  Every
+// path visits a superset of the cells the reference visits and applies the
+// reference's per-point box test to each, in the same order.
+template <int D, int OD>
+__device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* __restrict__ counts, int bx, int gx) {
+    constexpr int d = D;
+    extern __shared__ float4 s_tab[];  // sin, cos, 1 - cos of k * side; then each warp's area
+    __shared__ int s_list[256];
+    __shared__ int s_count;
     const int K = g.table_k, TW = 2 * K + 1;
-    const int i = bx * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const bool valid = i < g.n;
-    const int iv = valid ? i : g.n - 1;  // lanes past n shadow the last point; their results are dropped
+    const bool tiled = tile_dims(D) && w.ctrl[kCtrlTiled] != 0;
+    const int t0 = tiled ? bx * blockDim.x + threadIdx.x : (((int)(threadIdx.x >> 5) * gx + bx) << 5) + lane;
+    const bool valid = t0 < g.n;
+    const int tv = valid ? t0 : g.n - 1;  // lanes past n shadow the last point; their results are dropped
+    const int i = tiled ? w.perm[tv] : tv;
     // the point and its warp's last violation bits are loaded before the
     // table's barrier, so their latency overlaps it (most warps late in a
     // run need nothing else)
-    float x[DM];
-    for (int l = 0; l < d; l++) x[l] = w.X[(size_t)l * g.ns + iv];
-    const unsigned wv_last = (w.warp_viol && (i & ~31) < g.n) ? w.warp_viol[i >> 5] : 0u;
-    for (int t = threadIdx.x; t < 3 * TW; t += blockDim.x) s_tab[t] = w.table[t];
-    if (bx == 0 && threadIdx.x == 0) {
-        const int it = w.ctrl[kCtrlIter];
-        w.stamps[4 * it + 1] = globaltimer();
+    float x[D];
+#pragma unroll
+    for (int l = 0; l < d; l++) x[l] = w.X[(size_t)l * g.ns + i];
+    const unsigned wv_last = tiled ? 0u : w.warp_viol[i >> 5];
+    for (int t = threadIdx.x; t < TW; t += blockDim.x)
+        s_tab[t] = make_float4(w.table[t], w.table[TW + t], w.table[2 * TW + t], 0.f);
+    const int it = w.ctrl[kCtrlIter];
+    if (threadIdx.x == 0) {
+        s_count = 0;
+        if (bx == 0) w.stamps[4 * it + 1] = globaltimer();
     }
     __syncthreads();
-    if ((i & ~31) >= g.n) return;  // whole warp beyond n
-    const float* Ts = s_tab;
-    const float* Tc = s_tab + TW;
-    const float* Tm = s_tab + 2 * TW;
-
-    const int it = w.ctrl[kCtrlIter];
-    int gi[DM];
-    int obase = 0;
-    for (int l = 0; l < d; l++) {
-        gi[l] = cell_dim(x[l], g);
-        if (l < g.od) obase += gi[l] * g.wpow[l];
-    }
-
-    // Incremental update: when no point of this warp has a moved point (old
-    // or new position) anywhere in its stencil region since the last update,
-    // every input of its update is unchanged, so the result is the same bit
-    // for bit: keep the position and the last violation bit.
-    const int zb = g.od < d ? gi[g.od] / g.zblk : 0;
-    const bool need_me = w.ctrl[kCtrlForce] != 0 || ((w.need[obase] >> zb) & 1ull) != 0;
-    // Xn equals X here unless this iteration rebuilt the grid (the grid check
-    // copied Xn into X; a rebuild reorders X only): a kept position is
-    // written back only after a rebuild (the control word is read where it
-    // is used, so nothing extra stays live over the walk)
-    // Without a rebuild the warp holds the same points as at its last update
-    // and its violation bits stand; a rebuild reorders the points, so the
-    // bits are gathered by original index and the warp's word rewritten.
-    if (!__any_sync(0xffffffffu, need_me)) {
-        unsigned vb = wv_last;
-        if (w.ctrl[kCtrlChanged] != 0 || !w.warp_viol) {
-            bool viol = false;
-            if (valid) {
-                for (int l = 0; l < d; l++) w.Xn[(size_t)l * g.ns + i] = x[l];
-                viol = w.viol_orig[w.orig[i]] != 0;
-            }
-            vb = __ballot_sync(0xffffffffu, viol);
-            if (lane == 0 && w.warp_viol) w.warp_viol[i >> 5] = vb;
-        }
-        if (lane == 0) {
-            if (w.warp_moved) w.warp_moved[i >> 5] = 0;
-            if (vb != 0) {
-                volatile int* f = w.ctrl + kCtrlFlag;
-                if (*f != 0) *f = 0;
-            }
-        }
-        return;
-    }
-    // Within a warp that recomputes, a lane whose own region is clean keeps
-    // its result too (same argument, per point): it does not walk when the
-    // lanes walk separately (lanes in several outer cells), where the walks
-    // of a warp's lanes run one after another.  The lane's need bit is read
-    // again where it is used, so nothing extra stays live over the walk.
-    auto lane_needs = [&]() {
-        return counts != nullptr || w.ctrl[kCtrlForce] != 0 ||
-               ((w.need[obase] >> (g.od < d ? gi[g.od] / g.zblk : 0)) & 1ull) != 0;
-    };
-    {
-        const unsigned vm = __ballot_sync(0xffffffffu, valid && (need_me || counts != nullptr));
-        if (lane == 0) atomicAdd(w.ctrl + kCtrlComputed, __popc(vm));
-    }
-
-    bool border = false;
-    Acc<D> a;
-    for (int l = 0; l < d; l++) {
-        border |= on_border_dim(x[l], g.side);
-        a.S[l] = 0.f;
-        a.Cm[l] = 0.f;
-    }
-    a.N = 0;
-    a.partial_in = 0;
-    a.tab_err = false;
-#ifdef EGG_UPDATE_STATS
-    for (int k = 0; k < kUStats; k++) a.st[k] = 0;
-    {
-        // every lane takes part in the vote (a full-mask vote by one lane never completes)
-        const int ob0 = __shfl_sync(0xffffffffu, obase, 0);
-        const bool uniform = __all_sync(0xffffffffu, obase == ob0);
-        if (lane == 0 && !uniform) a.st[kUsLaneWarps] = 1;
-    }
-#endif
-    const int own = w.cell_of[iv];
-    const int own_cnt = w.cell_start[own + 1] - w.cell_start[own];
-
-#ifdef EGG_UPDATE_STATS
-    const long long t_walk0 = clock64();
-#endif
-#ifdef EGG_UPDATE_STATS
-    const bool ls_warp = a.st[kUsLaneWarps] == 0;  // meaningful in lane 0, which counts
-    for_candidates(g, w, gi, obase, lane, d, lane_needs, [&](int c) {
-        const long long tv = clock64();
-        visit_cell<D>(g, w, c, x, gi, a, Ts, Tc, Tm, K, TW);
-        if (lane == 0 && ls_warp) {
-            a.st[kUsWarpVisits] += 1;
-            a.st[kUsCyclesVisits] += (unsigned)(clock64() - tv);
-        }
-    });
-#else
-    for_candidates(g, w, gi, obase, lane, d, lane_needs,
-                   [&](int c) { visit_cell<D>(g, w, c, x, gi, a, Ts, Tc, Tm, K, TW); });
-#endif
-#ifdef EGG_UPDATE_STATS
-    {
-        const long long dt = clock64() - t_walk0;
-        const long long warp_dt = __reduce_max_sync(0xffffffffu, (unsigned)min(dt, 0x7fffffffLL));
-        if (lane == 0) a.st[a.st[kUsLaneWarps] ? kUsCyclesLane : kUsCyclesShared] += (unsigned)warp_dt;
-    }
-#endif
-
-    const bool walk = lane_needs();
-    const int N = a.N;
-    const float fN = (float)N;
-    bool moved = false;
-    int onew = 0, zbnew = 0;
-    if (valid && !walk) {
-        if (w.ctrl[kCtrlChanged] != 0)
-            for (int l = 0; l < d; l++) w.Xn[(size_t)l * g.ns + i] = x[l];
-    } else if (valid) {
-        for (int l = 0; l < d; l++) {
-            const float corner = __fmul_rn((float)gi[l], g.side);
-            const float phi = x[l] - corner;
-            float sp, cp;
-            sincosf(phi, &sp, &cp);
-            const float A = cp * a.S[l] - sp * (fN - a.Cm[l]);
-            const float xn = x[l] + A / fN;
-            w.Xn[(size_t)l * g.ns + i] = xn;
-            moved |= __float_as_uint(xn) != __float_as_uint(x[l]);
-            if (l < g.od) onew += cell_dim(xn, g) * g.wpow[l];
-            if (l == g.od) zbnew = cell_dim(xn, g) / g.zblk;
-        }
-        if (counts) counts[i] = N;
-    }
-
-    // convergence flag, EGG_SynC.cu:706-709.  half_count <= N - partial_in,
-    // so a border point with neighbours in a partial cell always violates.
     bool viol = false;
-    if (valid && !walk) {
-        viol = (w.ctrl[kCtrlChanged] != 0 || !w.warp_viol) ? w.viol_orig[w.orig[i]] != 0
-                                                           : ((w.warp_viol[i >> 5] >> lane) & 1u) != 0;
-    } else if (valid) {
-        if (!border) viol = (N != own_cnt);
-        else if (a.partial_in > 0) viol = true;
-        else if (N == own_cnt) viol = false;
-        else {
-            viol = (N != half_count<D>(g, w, x, gi, obase, own, own_cnt));
-            EGG_STAT(a, kUsHalfCount, 1);
-        }
-        w.viol_orig[w.orig[i]] = viol ? 1 : 0;
-        if (moved) {
-            unsigned long long* dcur = w.dirty[it & 1];
-            atomicOr(dcur + obase, 1ull << zb);
-            atomicOr(dcur + onew, 1ull << zbnew);
-        }
-    }
-    // the warps whose points moved: the next grid check reads only those
-    const bool warp_mv = __any_sync(0xffffffffu, moved);
-    if (lane == 0 && w.warp_moved) w.warp_moved[i >> 5] = warp_mv ? 1 : 0;
-    const unsigned vb = __ballot_sync(0xffffffffu, viol);
-    if (lane == 0) {
-        if (w.warp_viol) w.warp_viol[i >> 5] = vb;
-        if (vb != 0) {
-            volatile int* f = w.ctrl + kCtrlFlag;
-            if (*f != 0) *f = 0;
-        }
-    }
-    if (a.tab_err) atomicOr(w.ctrl + kCtrlStatus, kErrTable);
-#ifdef EGG_UPDATE_STATS
-    if (valid && walk) {
-        a.st[kUsPoints] += 1;
-        a.st[kUsNeighbors] += N;
-    } else {
-        // shadow lanes, and lanes that kept their result (their lockstep
-        // visits are not work of the update)
-        for (int k = 0; k < kUStats; k++)
-            if (k != kUsLaneWarps && k != kUsCyclesShared && k != kUsCyclesLane && k != kUsWarpVisits &&
-                k != kUsCyclesVisits && k != kUsWalkSteps)
-                a.st[k] = 0;
-    }
-    for (int k = 0; k < kUStats; k++) {
-        unsigned long long v = a.st[k];
+    if ((t0 & ~31) < g.n) {  // uniform across the warp
+        bool bad = false;  // the point violates
+        int gi[D];
+        int obase = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && v) atomicAdd(w.ustats + k, v);
-    }
+        for (int l = 0; l < d; l++) {
+            gi[l] = cell_dim(x[l], g);
+            if (l < g.od) obase += gi[l] * g.wpow[l];
+        }
+        // Incremental update: when no point of a point's stencil region moved
+        // (old or new position) since the last update, every input of its
+        // update is unchanged, so the result is the same bit for bit: it keeps
+        // the position and the last violation bit.  The need bit is read again
+        // where it is used, so nothing extra stays live over the walk.
+        auto zblk_of = [&]() {
+            int z = 0;
+#pragma unroll
+            for (int l = 0; l < d; l++)
+                if (l == g.od) z = gi[l] / g.zblk;
+            return z;
+        };
+        auto needs = [&]() {
+            return valid && (counts != nullptr || w.ctrl[kCtrlForce] != 0 || ((w.need[obase] >> zblk_of()) & 1ull) != 0);
+        };
+        const unsigned nm = __ballot_sync(0xffffffffu, needs());
+        Acc<D> a;
+#pragma unroll
+        for (int l = 0; l < d; l++) a.S[l] = a.Cm[l] = 0.f;
+        a.N = a.partial_in = 0;
+#ifdef EGG_UPDATE_STATS
+        for (int k = 0; k < kUStats; k++) a.st[k] = 0;
+        const long long t_walk0 = clock64();
 #endif
+        bool done = false;  // the lanes that need it have their sums (uniform across the warp)
+        if (nm) {
+            if (lane == 0) atomicAdd(w.ctrl + kCtrlComputed, __popc(nm));
+            ulonglong2* sh = reinterpret_cast<ulonglong2*>(s_tab + TW) + (threadIdx.x >> 5) * warp_words(D);
+            done = walk_union<D, OD>(g, w, x, gi, needs(), tiled, a, s_tab, K, sh, lane);
+            if (!done && needs()) s_list[atomicAdd(&s_count, 1)] = i;
+        }
+#ifdef EGG_UPDATE_STATS
+        if (nm) {
+            const long long dt = clock64() - t_walk0;
+            const long long warp_dt = __reduce_max_sync(0xffffffffu, (unsigned)min(dt, 0x7fffffffLL));
+            if (lane == 0) a.st[done ? kUsCyclesShared : kUsCyclesLane] += (unsigned)warp_dt;
+            if (lane == 0 && !done) a.st[kUsLaneWarps] = 1;
+        }
+#endif
+        bool moved = false;
+        if (valid && !needs()) {
+            // Xn equals X unless this iteration rebuilt the grid (the grid
+            // check copied Xn into X; a rebuild reorders X only).  A rebuild
+            // reorders the points, and in tile order the storage warps' words
+            // are not kept up: then the violation bit goes by original index.
+            if (w.ctrl[kCtrlChanged] != 0)
+                for (int l = 0; l < d; l++) w.Xn[(size_t)l * g.ns + i] = x[l];
+            bad = tiled || w.ctrl[kCtrlChanged] != 0 ? w.viol_orig[w.orig[i]] != 0 : ((wv_last >> lane) & 1u) != 0;
+        } else if (valid && done) {
+            const int N = a.N;
+            const float fN = (float)N;
+            bool border = false;
+            int onew = 0, zbnew = 0;
+#pragma unroll
+            for (int l = 0; l < d; l++) {
+                border |= on_border_dim(x[l], g.side);
+                const float corner = __fmul_rn((float)gi[l], g.side);
+                const float phi = x[l] - corner;
+                float sp, cp;
+                sincosf(phi, &sp, &cp);
+                const float A = cp * a.S[l] - sp * (fN - a.Cm[l]);
+                const float xn = x[l] + A / fN;
+                w.Xn[(size_t)l * g.ns + i] = xn;
+                moved |= __float_as_uint(xn) != __float_as_uint(x[l]);
+                if (l < g.od) onew += cell_dim(xn, g) * g.wpow[l];
+                if (l == g.od) zbnew = cell_dim(xn, g) / g.zblk;
+            }
+            if (counts) counts[i] = N;
+            // convergence flag, EGG_SynC.cu:706-709.  half_count <= N -
+            // partial_in, so a border point with neighbours in a partial cell
+            // always violates.
+            const int own = w.cell_of[i];
+            const int own_cnt = w.cell_start[own + 1] - w.cell_start[own];
+            if (!border) bad = (N != own_cnt);
+            else if (a.partial_in > 0) bad = true;
+            else if (N == own_cnt) bad = false;
+            else {
+                bad = (N != half_count<D>(g, w, x, gi, obase, own, own_cnt));
+                EGG_STAT(a, kUsHalfCount, 1);
+            }
+            w.viol_orig[w.orig[i]] = bad ? 1 : 0;
+            if (moved) {
+                unsigned long long* dcur = w.dirty[it & 1];
+                atomicOr(dcur + obase, 1ull << zblk_of());
+                atomicOr(dcur + onew, 1ull << zbnew);
+            }
+            EGG_STAT(a, kUsPoints, 1);
+            EGG_STAT(a, kUsNeighbors, N);
+        }
+        // the storage warps whose points moved: the next grid check reads only
+        // those (in tile order the cell-sums kernels of this iteration cleared
+        // the marks; a listed point adds its own mark and bit below)
+        const unsigned vb = __ballot_sync(0xffffffffu, bad), mb = __ballot_sync(0xffffffffu, moved);
+        viol |= bad;
+        if (tiled) {
+            if (moved) w.warp_moved[i >> 5] = 1;
+        } else if (lane == 0) {
+            w.warp_moved[i >> 5] = mb != 0;
+            if (nm || w.ctrl[kCtrlChanged] != 0) w.warp_viol[i >> 5] = vb;
+        }
+#ifdef EGG_UPDATE_STATS
+        for (int k = 0; k < kUStats; k++) {
+            unsigned long long v = a.st[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0 && v) atomicAdd(w.ustats + k, v);
+        }
+#endif
+    }
+    __syncthreads();
+    const int todo = s_count;
+    if (todo) {
+        float* area = reinterpret_cast<float*>(s_tab + TW) + (threadIdx.x >> 5) * (4 * warp_words(D));
+        viol |= update_listed_points<D, true>(g, w, counts, s_tab, area, s_list, todo, !tiled);
+    }
+    if (__any_sync(0xffffffffu, viol) && lane == 0) {
+        volatile int* f = w.ctrl + kCtrlFlag;
+        if (*f != 0) *f = 0;
+    }
 }
 
-template <int D>
-__global__ void __launch_bounds__(128) k_update(Geom g, Work w, int* __restrict__ counts) {
-    update_body<D>(g, w, counts, blockIdx.x);
+template <int D, int OD>
+__global__ void __launch_bounds__(128, update_min_blocks(D, 128)) k_update(Geom g, Work w, int* __restrict__ counts) {
+    update_body<D, OD>(g, w, counts, blockIdx.x, gridDim.x);
 }
 
 template <int D, int T>
-__global__ void __launch_bounds__(T) kb_update(BatchArgs B) {
-    batch_for(B, [&](const Geom& g, const Work& w, int bx, int) { update_body<D>(g, w, nullptr, bx); });
+__global__ void __launch_bounds__(T, update_min_blocks(D, T)) kb_update(BatchArgs B) {
+    batch_for(B, [&](const Geom& g, const Work& w, int bx, int gx) { update_body<D, 0>(g, w, nullptr, bx, gx); });
 }
-
-#define EGG_DISPATCH_D(d, KERNEL, ...)                \
-    switch (d) {                                      \
-        case 1: KERNEL<1> __VA_ARGS__; break;         \
-        case 2: KERNEL<2> __VA_ARGS__; break;         \
-        case 3: KERNEL<3> __VA_ARGS__; break;         \
-        case 4: KERNEL<4> __VA_ARGS__; break;         \
-        case 5: KERNEL<5> __VA_ARGS__; break;         \
-        case 6: KERNEL<6> __VA_ARGS__; break;         \
-        case 8: KERNEL<8> __VA_ARGS__; break;         \
-        case 16: KERNEL<16> __VA_ARGS__; break;       \
-        default: KERNEL<0> __VA_ARGS__; break;        \
-    }
 
 // need[] (zeroed by the grid-build check of this iteration) receives, over
 // the stencil of every outer cell that the previous update marked dirty, the
@@ -574,35 +845,47 @@ void launch_need(const Exec& ex, cudaStream_t st) {
         k_need<<<ex.blocks(kShapeCapOuter, 256), 256, 0, st>>>(*ex.g, *ex.w);
 }
 
-#define EGG_DISPATCH_DT(d, KERNEL, T, ...)            \
-    switch (d) {                                      \
-        case 1: KERNEL<1, T> __VA_ARGS__; break;      \
-        case 2: KERNEL<2, T> __VA_ARGS__; break;      \
-        case 3: KERNEL<3, T> __VA_ARGS__; break;      \
-        case 4: KERNEL<4, T> __VA_ARGS__; break;      \
-        case 5: KERNEL<5, T> __VA_ARGS__; break;      \
-        case 6: KERNEL<6, T> __VA_ARGS__; break;      \
-        case 8: KERNEL<8, T> __VA_ARGS__; break;      \
-        case 16: KERNEL<16, T> __VA_ARGS__; break;    \
-        default: KERNEL<0, T> __VA_ARGS__; break;     \
-    }
-
 template <int T>
 void launch_update_batch(const Exec& ex, size_t smem, cudaStream_t st) {
-    const int shape = T == 64 ? kShapeN64 : (T == 128 ? kShapeN128 : kShapeN256);
-    EGG_DISPATCH_DT(ex.d, kb_update, T, <<<ex.blocks(shape, T), T, smem, st>>>(ex.args(shape)));
+    const int shape = T == 128 ? kShapeN128 : kShapeN256;
+    // at most 36 KB (256 threads) beside the descriptors' static 10 KB: below the 48 KB that need no opt-in
+    auto go = [&](auto kernel) { kernel<<<ex.blocks(shape, T), T, smem, st>>>(ex.args(shape)); };
+    switch (ex.d) {
+        case 1: go(kb_update<1, T>); break;
+        case 2: go(kb_update<2, T>); break;
+        case 3: go(kb_update<3, T>); break;
+        case 4: go(kb_update<4, T>); break;
+        default: break;  // d > 4: launch_update_wide
+    }
 }
 
 void launch_update(const Exec& ex, int* counts, cudaStream_t st) {
-    const size_t smem = sizeof(float) * 3 * (2 * ex.table_k() + 1);
+    // below the tile order's size too few warps of 32 points are at hand to
+    // fill the chip: a warp per point (10k x 2D)
+    if (ex.d > 4 || (!ex.batch() && ex.g->point_walk)) {
+        launch_update_wide(ex, counts, st);
+        return;
+    }
+    const size_t stage = (size_t)warp_words(ex.d);  // 16-byte words per warp (point walks take less)
+    const size_t smem = 16 * ((2 * (size_t)ex.table_k() + 1) + stage * (ex.update_threads() / 32));
     if (ex.batch()) {
         switch (ex.update_threads()) {
-            case 64: launch_update_batch<64>(ex, smem, st); break;
-            case 256: launch_update_batch<256>(ex, smem, st); break;
-            default: launch_update_batch<128>(ex, smem, st); break;
+            case 128: launch_update_batch<128>(ex, smem, st); break;
+            default: launch_update_batch<256>(ex, smem, st); break;
         }
     } else {
-        EGG_DISPATCH_D(ex.d, k_update, <<<ex.blocks(kShapeN128, 128), 128, smem, st>>>(*ex.g, *ex.w, counts));
+        // two outer dimensions are what n points give (width^2 <= n < width^3)
+        // at nearly every eps in use: known to the compiler for d = 2, 3, 4
+        const bool od2 = ex.g->od == 2;
+        const int blocks = ex.blocks(kShapeN128, 128);
+        auto go = [&](auto kernel) { kernel<<<blocks, 128, smem, st>>>(*ex.g, *ex.w, counts); };
+        switch (ex.d) {
+            case 1: go(k_update<1, 0>); break;
+            case 2: od2 ? go(k_update<2, 2>) : go(k_update<2, 0>); break;
+            case 3: od2 ? go(k_update<3, 2>) : go(k_update<3, 0>); break;
+            case 4: od2 ? go(k_update<4, 2>) : go(k_update<4, 0>); break;
+            default: break;  // d > 4: launch_update_wide
+        }
     }
 }
 
