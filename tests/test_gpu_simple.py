@@ -69,3 +69,22 @@ def test_wrapper_shapes_and_device_input(gpu):
     lab, info = simple_sync(torch.from_numpy(X).to(gpu), eps)
     assert C.shape == (len(X),) and itr.shape == (info["iterations"],) and stages.shape == (6,)
     assert np.array_equal(C.numpy().astype(np.int32), lab)
+
+
+@pytest.mark.parametrize("n,d", [(1, 2), (2, 3), (31, 2), (33, 5), (255, 8), (257, 3), (300, 7), (129, 16), (70, 31),
+                                 (90, 32), (65, 64)])
+def test_first_update_at_tile_edges(oracle, n, d):
+    """Odd sizes around the 32-point steps and the staged tiles, one to three
+    registers of components per lane: the update within 1e-5 of the FP64
+    oracle (as above), duplicates included."""
+    rng = np.random.default_rng(n + d)
+    X = rng.uniform(0.3, 0.7, (n, d)).astype(np.float32)
+    X[n // 2:] = X[: n - n // 2] + np.float32(0.01) * rng.standard_normal((n - n // 2, d)).astype(np.float32)
+    X[n - 1] = X[0]
+    eps = 0.08 * float(np.sqrt(d))
+    P = np.empty_like(X)
+    lab, info = simple_sync(X, eps, max_iter=1, positions_out=P)
+    xs, cnt = oracle.update_sample(X, eps, np.arange(n, dtype=np.int32))
+    assert np.abs(P - xs).max() <= 1e-5
+    assert abs(info["r_local"] - oracle.order_parameter(X, eps)) <= 1e-5
+    assert info["n_clusters"] == len(set(lab[lab >= 0].tolist()))
