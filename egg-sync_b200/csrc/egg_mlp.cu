@@ -16,10 +16,9 @@
 //              shared memory, FP32 accumulators in TMEM); a CTA owns
 //              128-point tiles, the next tile's features arrive by cp.async
 //              while the current one runs.
-//   training   FP32 kernels: tiled SGEMM, bias/ReLU, ReLU backward, column
-//              sums (fixed order), MSE gradient, Adam.  The gradient of one
-//              batch is exported (egg_mlp_grad) so that tests can check it
-//              against a CPU computation.
+//   training   FP32 kernels, fused per layer, every sum in a fixed order.  The
+//              gradient of one batch is exported (egg_mlp_grad) so that tests
+//              can check it against a CPU computation.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -463,128 +462,359 @@ __global__ void k_apply(FGrid G, float* X, size_t ns, int n, const float* __rest
 // ---------------------------------------------------------------------------
 // training (FP32)
 // ---------------------------------------------------------------------------
-// C[M][N] = op(A)[M][K] . op(B)[K][N] (+ beta C); op(A)[m][k] = TA ? A[k][m] : A[m][k]
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float* __restrict__ A, int lda,
-                                               const float* __restrict__ B, int ldb, float* __restrict__ C, int ldc,
-                                               float beta) {
-    __shared__ float As[16][65];
-    __shared__ float Bs[16][65];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
+// One step is five launches: the two hidden layers forward (bias and ReLU in
+// the epilogue, the batch's rows read through the shuffled index), the head
+// (layer 3, loss, its gradient and the masked gradient of the second hidden
+// layer), the gradient of the first hidden layer, and all weight and bias
+// gradients with Adam in their epilogue.  Every sum runs over its index in
+// ascending order in one FP32 chain, so a value does not depend on the tiles.
+// At the batches in use the chains' latency is the floor: 2,048 rows times
+// four cycles is 4 us for a weight gradient, which many small tiles reach and
+// a few large ones do not (2 to 6 blocks of 64 x 64 before: 100 to 400 us, and
+// 100 us for a bias gradient by one thread per column).  A step of 2,048 rows
+// took 1,500 us of kernels, now 84 (two of 12 forward, 7 head, 12, 41).
+
+// two multiply-adds at once, each rounded as fmaf
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long dup2(float v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ void split2(unsigned long long v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+constexpr int kRowTile = 32, kColTile = 64, kKTile = 32;  // layer products: 128 threads, 4 x 4 values each
+
+// C[m][n] = epilogue(sum_k A[row(m)][k] B[k][n]) for n < kHidden, row(m) =
+// idx ? idx[m] : m.  BT: B[k][n] is stored as B[n][k] (kHidden x K).  With
+// bias: + bias[n], then ReLU.  With gate: the value where gate[m][n] > 0,
+// else 0.  Rows of A are lda floats, 16-byte aligned; K <= lda.
+template <bool BT>
+__global__ void __launch_bounds__(128) k_layer(int M, int K, const float* __restrict__ A, int lda,
+                                               const int* __restrict__ idx, const float* __restrict__ B,
+                                               const float* __restrict__ bias, const float* __restrict__ gate,
+                                               float* __restrict__ C) {
+    __shared__ __align__(16) float As[kKTile][kRowTile + 4];  // [k][m]
+    __shared__ __align__(16) float Bs[kKTile][kColTile + 4];  // [k][n]
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int m0 = blockIdx.y * kRowTile, n0 = blockIdx.x * kColTile;
+    // loads of one k-tile: A 32 rows x 8 float4 (two per thread), B 512 float4 (four per thread)
+    const float* arow[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int r = m0 + (tid >> 3) + 16 * i;
+        arow[i] = r < M ? A + (size_t)(idx ? idx[r] : r) * lda : nullptr;
+    }
+    const int ak = (tid & 7) * 4;
+    float4 ra[2], rb[4];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int k = k0 + ak;
+            if (arow[i] && k < K) {
+                v = __ldg(reinterpret_cast<const float4*>(arow[i] + k));
+                if (k + 1 >= K) v.y = 0.f;  // the row's padding is not part of it
+                if (k + 2 >= K) v.z = 0.f;
+                if (k + 3 >= K) v.w = 0.f;
+            }
+            ra[i] = v;
+        }
+#pragma unroll
         for (int i = 0; i < 4; i++) {
-            const int idx = threadIdx.x + 256 * i;
-            const int kk = TA ? idx / 64 : idx % 16, mm = TA ? idx % 64 : idx / 16;
-            const int m = m0 + mm, k = k0 + kk;
-            float v = 0.f;
-            if (m < M && k < K) v = TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-            As[kk][mm] = v;
-            const int kb = TB ? idx % 16 : idx / 64, nn = TB ? idx / 16 : idx % 64;
-            const int nb = n0 + nn, kb2 = k0 + kb;
-            float u = 0.f;
-            if (nb < N && kb2 < K) u = TB ? B[(size_t)nb * ldb + kb2] : B[(size_t)kb2 * ldb + nb];
-            Bs[kb][nn] = u;
+            const int t = tid + 128 * i;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (BT) {  // n = t / 8, four k
+                const int n = n0 + (t >> 3), k = k0 + (t & 7) * 4;
+                if (k < K) v = __ldg(reinterpret_cast<const float4*>(B + (size_t)n * K + k));
+            } else {  // k = t / 16, four n
+                const int k = k0 + (t >> 4), n = n0 + (t & 15) * 4;
+                if (k < K) v = __ldg(reinterpret_cast<const float4*>(B + (size_t)k * kHidden + n));
+            }
+            rb[i] = v;
+        }
+    };
+    unsigned long long acc[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc[i][0] = acc[i][1] = 0ull;
+    fetch(0);
+    for (int k0 = 0; k0 < K; k0 += kKTile) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int m = (tid >> 3) + 16 * i;
+            As[ak][m] = ra[i].x;
+            As[ak + 1][m] = ra[i].y;
+            As[ak + 2][m] = ra[i].z;
+            As[ak + 3][m] = ra[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int t = tid + 128 * i;
+            if (BT) {
+                const int n = t >> 3, k = (t & 7) * 4;
+                Bs[k][n] = rb[i].x;
+                Bs[k + 1][n] = rb[i].y;
+                Bs[k + 2][n] = rb[i].z;
+                Bs[k + 3][n] = rb[i].w;
+            } else {
+                *reinterpret_cast<float4*>(&Bs[t >> 4][(t & 15) * 4]) = rb[i];
+            }
         }
         __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
+        if (k0 + kKTile < K) fetch(k0 + kKTile);
+#pragma unroll 8
+        for (int k = 0; k < kKTile; k++) {
+            const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&Bs[k][tx * 4]);
+            const unsigned long long av[4] = {dup2(a.x), dup2(a.y), dup2(a.z), dup2(a.w)};
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                a[i] = As[kk][ty + 16 * i];
-                b[i] = Bs[kk][tx + 16 * i];
+                acc[i][0] = fma2(av[i], b.x, acc[i][0]);
+                acc[i][1] = fma2(av[i], b.y, acc[i][1]);
             }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         __syncthreads();
     }
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) {
-            const int m = m0 + ty + 16 * i, nn = n0 + tx + 16 * j;
-            if (m < M && nn < N) {
-                float* c = C + (size_t)m * ldc + nn;
-                *c = acc[i][j] + (beta != 0.f ? beta * *c : 0.f);
-            }
+    const int n = n0 + tx * 4;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int m = m0 + ty * 4 + i;
+        if (m >= M) break;
+        float v[4];
+        split2(acc[i][0], v[0], v[1]);
+        split2(acc[i][1], v[2], v[3]);
+        if (bias) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = fmaxf(v[j] + __ldg(bias + n + j), 0.f);
         }
-}
-
-__global__ void k_bias_act(float* H, int M, int N, const float* __restrict__ b, int relu) {
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)M * N;
-         t += (size_t)gridDim.x * blockDim.x) {
-        const float v = H[t] + b[t % N];
-        H[t] = relu ? fmaxf(v, 0.f) : v;
+        if (gate) {
+            const float4 h = __ldg(reinterpret_cast<const float4*>(gate + (size_t)m * kHidden + n));
+            v[0] = h.x > 0.f ? v[0] : 0.f;
+            v[1] = h.y > 0.f ? v[1] : 0.f;
+            v[2] = h.z > 0.f ? v[2] : 0.f;
+            v[3] = h.w > 0.f ? v[3] : 0.f;
+        }
+        *reinterpret_cast<float4*>(C + (size_t)m * kHidden + n) = make_float4(v[0], v[1], v[2], v[3]);
     }
 }
 
-__global__ void k_relu_back(float* dH, const float* __restrict__ H, size_t cnt) {
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < cnt; t += (size_t)gridDim.x * blockDim.x)
-        if (!(H[t] > 0.f)) dH[t] = 0.f;
-}
-
-// out[n] = sum_m X[m][n], each column summed in row order
-__global__ void k_colsum(const float* __restrict__ X, int M, int N, float* out) {
-    const int nn = blockIdx.x * blockDim.x + threadIdx.x;
-    if (nn >= N) return;
-    float s = 0.f;
-    for (int m = 0; m < M; m++) s += X[(size_t)m * N + nn];
-    out[nn] = s;
-}
-
-// dY = 2 (Y - T) / (M * N); per-block partial sums of (Y - T)^2
-__global__ void k_mse(const float* __restrict__ Y, const float* __restrict__ T, int M, int N, float* dY,
-                      double* partial) {
-    __shared__ double s[256];
-    double acc = 0.0;
-    const float scale = 2.f / ((float)M * (float)N);
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)M * N;
-         t += (size_t)gridDim.x * blockDim.x) {
-        const float e = Y[t] - T[t];
-        dY[t] = scale * e;
-        acc += (double)e * e;
+// Layer 3 and the loss: y = h2 w3 + b3, e = y - t, dy = 2 e / (M D); the
+// gradient of the second hidden layer behind its ReLU, dh2 = (dy w3^T) where
+// h2 > 0; per block the sum of e^2.
+constexpr int kHeadRows = 16, kHeadBlocks = 256;
+template <int D>
+__global__ void __launch_bounds__(kHidden) k_head(int M, const float* __restrict__ H2, const float* __restrict__ T,
+                                                  const int* __restrict__ idx, const float* __restrict__ w3,
+                                                  const float* __restrict__ b3, float* __restrict__ dY,
+                                                  float* __restrict__ dH2, double* __restrict__ loss) {
+    __shared__ float s_w[kHidden * D];
+    __shared__ float s_h[kHeadRows][kHidden + 1];
+    __shared__ float s_dy[kHeadRows][D];
+    __shared__ double s_l[kHeadRows * D];
+    const int tid = threadIdx.x;
+    for (int k = tid; k < kHidden * D; k += kHidden) s_w[k] = w3[k];
+    const float scale = 2.f / ((float)M * (float)D);
+    double l2 = 0.0;
+    for (int r0 = blockIdx.x * kHeadRows; r0 < M; r0 += gridDim.x * kHeadRows) {
+        const int rows = min(kHeadRows, M - r0);
+#pragma unroll 8
+        for (int r = 0; r < rows; r++) s_h[r][tid] = __ldg(H2 + (size_t)(r0 + r) * kHidden + tid);
+        __syncthreads();
+        if (tid < rows * D) {
+            const int r = tid / D, c = tid - r * D;
+            float y = 0.f;
+#pragma unroll 16
+            for (int k = 0; k < kHidden; k++) y = fmaf(s_h[r][k], s_w[k * D + c], y);
+            const float e = y + __ldg(b3 + c) - __ldg(T + (size_t)(idx ? idx[r0 + r] : r0 + r) * D + c);
+            const float dy = scale * e;
+            s_dy[r][c] = dy;
+            dY[(size_t)(r0 + r) * D + c] = dy;
+            l2 += (double)e * e;
+        }
+        __syncthreads();
+        for (int r = 0; r < rows; r++) {
+            float v = 0.f;
+#pragma unroll
+            for (int c = 0; c < D; c++) v = fmaf(s_dy[r][c], s_w[tid * D + c], v);
+            dH2[(size_t)(r0 + r) * kHidden + tid] = s_h[r][tid] > 0.f ? v : 0.f;
+        }
+        __syncthreads();
     }
-    s[threadIdx.x] = acc;
+    if (tid < kHeadRows * D) s_l[tid] = l2;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+    if (tid == 0) {
+        double sum = 0.0;
+        for (int k = 0; k < kHeadRows * D; k++) sum += s_l[k];
+        loss[blockIdx.x] = sum;
+    }
+}
+
+// The weight and bias gradients of all layers, each complete in one block:
+// dW[f][n] = sum over the rows of A[row][f] dY[r][n], db[n] = sum of dY[r][n].
+// Hidden layers: 8 f x 32 n per block, two n per thread; layer 3: 16 f x D.
+struct GradArgs {
+    int M, F, D, lda;
+    const float *X, *H1, *H2, *dH1, *dH2, *dY;
+    const int* idx;
+    float* p;  // parameters (Adam) or gradients (m == nullptr): w1 b1 w2 b2 w3 b3
+    float *m, *v;
+    float lr, c1, c2;  // beta1 0.9, beta2 0.999
+};
+constexpr int kGradRows = 64;  // rows staged at a time
+
+__device__ __forceinline__ void put_grad(const GradArgs& a, size_t t, float g) {
+    if (!a.m) {
+        a.p[t] = g;
+        return;
+    }
+    const float b1 = 0.9f, b2 = 0.999f;
+    a.m[t] = b1 * a.m[t] + (1.f - b1) * g;
+    a.v[t] = b2 * a.v[t] + (1.f - b2) * g * g;
+    a.p[t] -= a.lr * (a.m[t] / a.c1) / (sqrtf(a.v[t] / a.c2) + 1e-8f);
+}
+
+constexpr int kGradStages = 4;  // tiles in flight (one ahead: 66 us a launch at 2,048 rows, three ahead: 41)
+
+// 16 bytes from global to shared memory; bytes < 16 fills the rest with zeros
+__device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(bytes)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(128) k_grads(GradArgs a) {
+    __shared__ __align__(16) float As[kGradStages][kGradRows][8];   // [row][f]
+    __shared__ __align__(16) float Bs[kGradStages][kGradRows][32];  // [row][n]
+    const int tid = threadIdx.x, M = a.M, F = a.F, D = a.D;
+    const int nb1 = (F + 7) / 8 * 4, nb2 = kHidden / 8 * 4;
+    int b = blockIdx.x;
+    const size_t base2 = (size_t)(F + 1) * kHidden, base3 = base2 + (size_t)(kHidden + 1) * kHidden;
+    if (b < nb1 + nb2) {
+        // a hidden layer's tile.  f past nf (the rows' padding) and rows past
+        // M (zeros) reach only values that are not stored, or add zero.
+        const bool first = b < nb1;
+        if (!first) b -= nb1;
+        const int f0 = b / 4 * 8, n0 = b % 4 * 32, nf = first ? F : kHidden;
+        const float* A = first ? a.X : a.H1;
+        const float* dY = first ? a.dH1 : a.dH2;
+        const int lda = first ? a.lda : kHidden;
+        const int* idx = first ? a.idx : nullptr;
+        const int f = tid >> 4, np = tid & 15;  // this thread's outputs: (f, 2 np), (f, 2 np + 1)
+        const int ar = tid >> 1, af = (tid & 1) * 4;  // its row and columns of the A tiles
+        const int tiles = (M + kGradRows - 1) / kGradRows;
+        // the A row of a tile yet to come is looked up a ring ahead of its copy
+        auto row_of = [&](int t) {
+            const int r = t * kGradRows + ar;
+            return r < M ? (idx ? __ldg(idx + r) : r) : -1;
+        };
+        int row = row_of(0);
+        auto issue = [&](int t) {
+            if (t < tiles) {
+                const int s = t % kGradStages;
+                const int cur = row;
+                row = row_of(t + 1);
+                cp16(&As[s][ar][af], A + (size_t)max(cur, 0) * lda + f0 + af, cur >= 0 ? 16 : 0);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int u = tid + 128 * i, r = t * kGradRows + (u >> 3);
+                    cp16(&Bs[s][u >> 3][(u & 7) * 4], dY + (size_t)min(r, M - 1) * kHidden + n0 + (u & 7) * 4,
+                         r < M ? 16 : 0);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        unsigned long long acc = 0ull, bias = 0ull;
+        const unsigned long long ones = dup2(1.f);
+#pragma unroll
+        for (int t = 0; t < kGradStages - 1; t++) issue(t);
+        for (int t = 0; t < tiles; t++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kGradStages - 2) : "memory");
+            __syncthreads();  // tile t has arrived; the one its successor replaces is read
+            issue(t + kGradStages - 1);
+            const int s = t % kGradStages;
+#pragma unroll 16
+            for (int r = 0; r < kGradRows; r++) {
+                const unsigned long long bv = *reinterpret_cast<const unsigned long long*>(&Bs[s][r][2 * np]);
+                acc = fma2(dup2(As[s][r][f]), bv, acc);
+                if (f0 == 0) bias = fma2(ones, bv, bias);  // 1 * b + bias: the plain sum
+            }
+        }
+        float g0, g1;
+        split2(acc, g0, g1);
+        const size_t base = first ? 0 : base2;
+        const int n = n0 + 2 * np;
+        if (f0 + f < nf) {
+            put_grad(a, base + (size_t)(f0 + f) * kHidden + n, g0);
+            put_grad(a, base + (size_t)(f0 + f) * kHidden + n + 1, g1);
+        }
+        if (f0 == 0 && f == 0) {
+            split2(bias, g0, g1);
+            put_grad(a, base + (size_t)nf * kHidden + n, g0);
+            put_grad(a, base + (size_t)nf * kHidden + n + 1, g1);
+        }
+        return;
+    }
+    // layer 3: 16 rows of w3 (and, in the first block, b3); the tiles lie in
+    // Bs (columns 0-15: H2, 16-18: dY) the same way
+    const int f0 = (b - nb1 - nb2) * 16;
+    const int f = tid & 15, c = tid >> 4;  // c < D: a weight; c == 4, f < D in the first block: a bias
+    const bool weight = c < D, bias = f0 == 0 && c == 4 && f < D;
+    const int tiles = (M + kGradRows - 1) / kGradRows;
+    float dy[2];
+    auto fetch_dy = [&](int t) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int u = tid + 128 * i;
+            dy[i] = u < kGradRows * D && t * kGradRows + u / D < M ? __ldg(a.dY + (size_t)t * kGradRows * D + u) : 0.f;
+        }
+    };
+    auto issue = [&](int t) {
+        if (t < tiles) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int u = tid + 128 * i, r = t * kGradRows + (u >> 2);
+                cp16(&Bs[t % kGradStages][u >> 2][(u & 3) * 4], a.H2 + (size_t)min(r, M - 1) * kHidden + f0 + (u & 3) * 4,
+                     r < M ? 16 : 0);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc = 0.f;
+#pragma unroll
+    for (int t = 0; t < kGradStages - 1; t++) issue(t);
+    fetch_dy(0);
+    for (int t = 0; t < tiles; t++) {
+        const int s = t % kGradStages;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int u = tid + 128 * i;
+            if (u < kGradRows * D) Bs[s][u / D][16 + u % D] = dy[i];
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(kGradStages - 2) : "memory");
         __syncthreads();
+        issue(t + kGradStages - 1);
+        if (t + 1 < tiles) fetch_dy(t + 1);
+        if (weight) {
+#pragma unroll 16
+            for (int r = 0; r < kGradRows; r++) acc = fmaf(Bs[s][r][f], Bs[s][r][16 + c], acc);
+        } else if (bias) {
+#pragma unroll 16
+            for (int r = 0; r < kGradRows; r++) acc += Bs[s][r][16 + f];
+        }
     }
-    if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
-}
-
-__global__ void k_adam(float* p, const float* __restrict__ gr, float* m, float* v, size_t cnt, float lr, float b1,
-                       float b2, float c1, float c2) {
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < cnt; t += (size_t)gridDim.x * blockDim.x) {
-        const float gg = gr[t];
-        m[t] = b1 * m[t] + (1.f - b1) * gg;
-        v[t] = b2 * v[t] + (1.f - b2) * gg * gg;
-        p[t] -= lr * (m[t] / c1) / (sqrtf(v[t] / c2) + 1e-8f);
-    }
-}
-
-__global__ void k_gather(const float* __restrict__ src, const int* __restrict__ idx, int rows, int cols,
-                         float* __restrict__ dst) {
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)rows * cols;
-         t += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(t / cols), c = (int)(t % cols);
-        dst[t] = src[(size_t)idx[r] * cols + c];
-    }
+    if (weight) put_grad(a, base3 + (size_t)(f0 + f) * D + c, acc);
+    if (bias) put_grad(a, base3 + (size_t)kHidden * D + f, acc);
 }
 
 int grid_for(size_t cnt, int threads = 256) {
     size_t b = (cnt + threads - 1) / threads;
     return (int)std::max<size_t>(1, std::min<size_t>(b, 148 * 16));
-}
-
-template <bool TA, bool TB>
-void sgemm(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc, float beta,
-           cudaStream_t st) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    k_sgemm<TA, TB><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, beta);
 }
 
 // parameter block on the device: w1 [F][H], b1 [H], w2 [H][H], b2 [H], w3 [H][D], b3 [D]
@@ -647,34 +877,42 @@ struct Scratch {
     }
 };
 
-// forward + backward of one batch X [M][F], T [M][D]; grads into G (same
-// layout as P); returns the batch's sum of squared errors on the device
-void batch_grad(const Params& P, const Params& G, const float* X, const float* T, int M, float* H1, float* H2,
-                float* Y, float* dY, float* dH2, float* dH1, double* partial, int nparts, cudaStream_t st) {
-    const int F = P.F, H = P.H, D = P.D;
-    sgemm<false, false>(M, H, F, X, F, P.w1(), H, H1, H, 0.f, st);
-    k_bias_act<<<grid_for((size_t)M * H), 256, 0, st>>>(H1, M, H, P.b1(), 1);
-    sgemm<false, false>(M, H, H, H1, H, P.w2(), H, H2, H, 0.f, st);
-    k_bias_act<<<grid_for((size_t)M * H), 256, 0, st>>>(H2, M, H, P.b2(), 1);
-    sgemm<false, false>(M, D, H, H2, H, P.w3(), D, Y, D, 0.f, st);
-    k_bias_act<<<grid_for((size_t)M * D), 256, 0, st>>>(Y, M, D, P.b3(), 0);
-    k_mse<<<nparts, 256, 0, st>>>(Y, T, M, D, dY, partial);
-    // layer 3
-    sgemm<true, false>(H, D, M, H2, H, dY, D, G.w3(), D, 0.f, st);
-    k_colsum<<<(D + 127) / 128, 128, 0, st>>>(dY, M, D, G.b3());
-    sgemm<false, true>(M, H, D, dY, D, P.w3(), D, dH2, H, 0.f, st);
-    k_relu_back<<<grid_for((size_t)M * H), 256, 0, st>>>(dH2, H2, (size_t)M * H);
-    // layer 2
-    sgemm<true, false>(H, H, M, H1, H, dH2, H, G.w2(), H, 0.f, st);
-    k_colsum<<<(H + 127) / 128, 128, 0, st>>>(dH2, M, H, G.b2());
-    sgemm<false, true>(M, H, H, dH2, H, P.w2(), H, dH1, H, 0.f, st);
-    k_relu_back<<<grid_for((size_t)M * H), 256, 0, st>>>(dH1, H1, (size_t)M * H);
-    // layer 1
-    sgemm<true, false>(F, H, M, X, F, dH1, H, G.w1(), H, 0.f, st);
-    k_colsum<<<(H + 127) / 128, 128, 0, st>>>(dH1, M, H, G.b1());
-}
+int head_blocks(int M) { return std::min(kHeadBlocks, (M + kHeadRows - 1) / kHeadRows); }
 
-constexpr int kLossParts = 64;
+// device arrays of one batch's forward and backward pass
+struct Batch {
+    int M = 0;
+    float *H1, *H2, *dH2, *dH1, *dY;
+    Batch(Scratch& S, int M_, int D) : M(M_) {
+        const size_t h = (size_t)M * kHidden;
+        H1 = S.get<float>(h);
+        H2 = S.get<float>(h);
+        dH2 = S.get<float>(h);
+        dH1 = S.get<float>(h);
+        dY = S.get<float>((size_t)M * D);
+    }
+};
+
+// forward + backward of the batch's rows X [.][lda] (columns past F ignored)
+// and T [.][D], through idx where given; the blocks' sums of squared errors
+// into loss[head_blocks(M)].  m == nullptr: the gradient into `out`; else one
+// Adam step on the parameters (out == P.base), whose last readers are done.
+void batch_step(const Params& P, const Batch& B, const float* X, int lda, const float* T, const int* idx, double* loss,
+                float* out, float* m, float* v, float lr, float c1, float c2, cudaStream_t st) {
+    const int M = B.M, F = P.F, H = kHidden, D = P.D;
+    const dim3 lg(H / kColTile, (M + kRowTile - 1) / kRowTile);
+    k_layer<false><<<lg, 128, 0, st>>>(M, F, X, lda, idx, P.w1(), P.b1(), nullptr, B.H1);
+    k_layer<false><<<lg, 128, 0, st>>>(M, H, B.H1, H, nullptr, P.w2(), P.b2(), nullptr, B.H2);
+    auto head = [&](auto kernel) {
+        kernel<<<head_blocks(M), H, 0, st>>>(M, B.H2, T, idx, P.w3(), P.b3(), B.dY, B.dH2, loss);
+    };
+    if (D == 1) head(k_head<1>);
+    else if (D == 2) head(k_head<2>);
+    else head(k_head<3>);
+    k_layer<true><<<lg, 128, 0, st>>>(M, H, B.dH2, H, nullptr, P.w2(), nullptr, B.H1, B.dH1);
+    GradArgs a{M, F, D, lda, X, B.H1, B.H2, B.dH1, B.dH2, B.dY, idx, out, m, v, lr, c1, c2};
+    k_grads<<<(F + 7) / 8 * 4 + H / 8 * 4 + H / 16, 128, 0, st>>>(a);
+}
 
 }  // namespace
 
@@ -801,6 +1039,15 @@ const float* to_device(const float* p, size_t cnt, Scratch& S, cudaStream_t st) 
     return d;
 }
 
+// the same, 16-byte aligned (the training kernels read rows in whole words)
+const float* to_device_aligned(const float* p, size_t cnt, Scratch& S, cudaStream_t st) {
+    const float* d = to_device(p, cnt, S, st);
+    if (((uintptr_t)d & 15) == 0) return d;
+    float* c = S.get<float>(cnt);
+    EGG_CHECK(cudaMemcpyAsync(c, d, 4 * cnt, cudaMemcpyDeviceToDevice, st));
+    return c;
+}
+
 }  // namespace
 
 int api_features(const float* x, int64_t n, int32_t d, float eps, float* feats) {
@@ -849,25 +1096,18 @@ int api_grad(const egg_mlp* m, const float* feats, const float* targets, int64_t
     cudaStream_t st = 0;
     Scratch S;
     const int F = feat_dim(m->d), fp = feat_pad(m->d), H = kHidden, D = m->d, M = (int)n;
-    // the host feature rows are padded to fp: compact them to F columns
-    const float* fd = to_device(feats, (size_t)n * fp, S, st);
-    float* X = S.get<float>((size_t)M * F);
-    EGG_CHECK(cudaMemcpy2DAsync(X, 4 * F, fd, 4 * fp, 4 * F, M, cudaMemcpyDeviceToDevice, st));
+    const float* X = to_device_aligned(feats, (size_t)n * fp, S, st);
     const float* T = to_device(targets, (size_t)n * D, S, st);
     Params P{F, H, D, S.get<float>(Params{F, H, D, nullptr}.count())};
     Params G{F, H, D, S.get<float>(P.count())};
     upload_params(*m, P, st);
-    float* H1 = S.get<float>((size_t)M * H);
-    float* H2 = S.get<float>((size_t)M * H);
-    float* Y = S.get<float>((size_t)M * D);
-    float* dY = S.get<float>((size_t)M * D);
-    float* dH2 = S.get<float>((size_t)M * H);
-    float* dH1 = S.get<float>((size_t)M * H);
-    double* part = S.get<double>(kLossParts);
-    batch_grad(P, G, X, T, M, H1, H2, Y, dY, dH2, dH1, part, kLossParts, st);
+    const Batch B(S, M, D);
+    const int parts = head_blocks(M);
+    double* part = S.get<double>(parts);
+    batch_step(P, B, X, fp, T, nullptr, part, G.base, nullptr, nullptr, 0.f, 1.f, 1.f, st);
     download_params(G, *grad, st);
-    std::vector<double> hp(kLossParts);
-    EGG_CHECK(cudaMemcpyAsync(hp.data(), part, 8 * kLossParts, cudaMemcpyDeviceToHost, st));
+    std::vector<double> hp(parts);
+    EGG_CHECK(cudaMemcpyAsync(hp.data(), part, 8 * (size_t)parts, cudaMemcpyDeviceToHost, st));
     EGG_CHECK(cudaStreamSynchronize(st));
     EGG_CHECK(cudaGetLastError());
     if (loss) {
@@ -888,33 +1128,24 @@ int api_train(egg_mlp* m, const float* feats, const float* targets, int64_t n, c
     cudaStream_t st = 0;
     Scratch S;
     const int F = feat_dim(m->d), fp = feat_pad(m->d), H = kHidden, D = m->d;
-    const float* fd = to_device(feats, (size_t)n * fp, S, st);
-    float* Xall = S.get<float>((size_t)n * F);
-    EGG_CHECK(cudaMemcpy2DAsync(Xall, 4 * F, fd, 4 * fp, 4 * F, n, cudaMemcpyDeviceToDevice, st));
+    const float* Xall = to_device_aligned(feats, (size_t)n * fp, S, st);
     const float* Tall = to_device(targets, (size_t)n * D, S, st);
     Params P{F, H, D, S.get<float>(Params{F, H, D, nullptr}.count())};
-    Params G{F, H, D, S.get<float>(P.count())};
     float* mom = S.get<float>(P.count());
     float* vel = S.get<float>(P.count());
     EGG_CHECK(cudaMemsetAsync(mom, 0, 4 * P.count(), st));
     EGG_CHECK(cudaMemsetAsync(vel, 0, 4 * P.count(), st));
     upload_params(*m, P, st);
     const int Bm = o->batch;
-    float* X = S.get<float>((size_t)Bm * F);
-    float* T = S.get<float>((size_t)Bm * D);
-    float* H1 = S.get<float>((size_t)Bm * H);
-    float* H2 = S.get<float>((size_t)Bm * H);
-    float* Y = S.get<float>((size_t)Bm * D);
-    float* dY = S.get<float>((size_t)Bm * D);
-    float* dH2 = S.get<float>((size_t)Bm * H);
-    float* dH1 = S.get<float>((size_t)Bm * H);
     const int nb = (int)(n / Bm);
     if (nb < 1) throw ArgError{EGG_ERR_ARG, "fewer samples than one batch"};
-    double* part = S.get<double>((size_t)kLossParts * nb);
+    const Batch B(S, Bm, D);
+    const int parts = head_blocks(Bm);
+    double* part = S.get<double>((size_t)parts * nb);
     int* idx = S.get<int>((size_t)nb * Bm);
     std::vector<int> perm(n);
     std::mt19937_64 rng((unsigned long long)o->seed);
-    std::vector<double> hp((size_t)kLossParts * nb);
+    std::vector<double> hp((size_t)parts * nb);
     int step = 0;
     for (int e = 0; e < o->epochs; e++) {
         std::iota(perm.begin(), perm.end(), 0);
@@ -922,15 +1153,12 @@ int api_train(egg_mlp* m, const float* feats, const float* targets, int64_t n, c
         EGG_CHECK(cudaMemcpyAsync(idx, perm.data(), 4 * (size_t)nb * Bm, cudaMemcpyHostToDevice, st));
         // cosine decay of the learning rate over the run
         for (int b = 0; b < nb; b++) {
-            k_gather<<<grid_for((size_t)Bm * F), 256, 0, st>>>(Xall, idx + (size_t)b * Bm, Bm, F, X);
-            k_gather<<<grid_for((size_t)Bm * D), 256, 0, st>>>(Tall, idx + (size_t)b * Bm, Bm, D, T);
-            batch_grad(P, G, X, T, Bm, H1, H2, Y, dY, dH2, dH1, part + (size_t)kLossParts * b, kLossParts, st);
             step++;
             const double frac = (double)(step - 1) / std::max(1, o->epochs * nb - 1);
             const float lr = (float)(o->lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(M_PI * frac))));
             const float c1 = 1.f - std::pow(0.9f, (float)step), c2 = 1.f - std::pow(0.999f, (float)step);
-            k_adam<<<grid_for(P.count()), 256, 0, st>>>(P.base, G.base, mom, vel, P.count(), lr, 0.9f, 0.999f, c1,
-                                                         c2);
+            batch_step(P, B, Xall, fp, Tall, idx + (size_t)b * Bm, part + (size_t)parts * b, P.base, mom, vel, lr, c1,
+                       c2, st);
         }
         EGG_CHECK(cudaMemcpyAsync(hp.data(), part, 8 * hp.size(), cudaMemcpyDeviceToHost, st));
         EGG_CHECK(cudaStreamSynchronize(st));
