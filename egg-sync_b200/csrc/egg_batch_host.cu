@@ -417,12 +417,15 @@ void set_tables(Plan& P, const Config& c) {
             bt->max_table_k = 0;
             bt->tile = false;
             bt->bytes = true;
+            bt->instances = bt->max_n = 0;
             for (int s = 0; s < kShapeCount; s++) bt->total[s] = 0;
             for (int i = 0; i < P.count; i++) {
                 if (P.geoms[i].d != gr.d) continue;
                 bt->max_passes = std::max(bt->max_passes, plan_count(P.geoms[i]));
                 bt->max_table_k = std::max(bt->max_table_k, P.geoms[i].table_k);
                 bt->tile = bt->tile || tile_capable(P.geoms[i]);
+                bt->instances++;
+                bt->max_n = std::max(bt->max_n, P.geoms[i].n);
                 bt->bytes = bt->bytes && byte_keys(P.geoms[i]);
                 for (int s = 0; s < kShapeCount; s++) bt->total[s] += shape_blocks(s, P.geoms[i]);
             }
@@ -488,6 +491,8 @@ std::vector<char> graph_key(const Plan& P) {
         put(&g.act.max_table_k, sizeof(int));
         put(&g.act.tile, sizeof(bool));
         put(&g.act.bytes, sizeof(bool));
+        put(&g.act.instances, sizeof(int));
+        put(&g.act.max_n, sizeof(int));
     }
     return k;
 }
@@ -599,7 +604,7 @@ cudaGraphExec_t get_graph(State& S, Plan& P, const Config& c) {
             // sort body: [sort, gate] -> IF(some instance wants a tile order) [tile order]
             if (e == cudaSuccess)
                 e = cond(gbody, hsort, prev, &ifs_sort, [&](cudaGraph_t sb) {
-                    if (!gex.tile) return seg(sb, nullptr, nullptr, [&] { enqueue_group(P, k, S.st, 1); });
+                    if (!gex.tile || gex.small_build()) return seg(sb, nullptr, nullptr, [&] { enqueue_group(P, k, S.st, 1); });
                     cudaGraphConditionalHandle ht;
                     cudaGraphNode_t last = nullptr, it_node = nullptr;
                     cudaError_t r = cudaGraphConditionalHandleCreate(&ht, sb, 0, 0);
@@ -843,8 +848,8 @@ int enqueue_prologue(State& S, Plan& P, int max_iter) {
 
 // kernels of one group's iteration: grid check, sort (radix passes, 4
 // tables), tile order (keys, 3 per pass), cell sums (2), need, update, extra check (3)
-int sort_launches(const Group& gr) { return 3 * gr.act.max_passes + 4; }
-int tile_launches(const Group& gr) { return gr.act.tile ? 1 + 3 * tile_passes(gr.d) : 0; }
+int sort_launches(const Group& gr) { return gr.act.max_n <= kSmallBuildN ? 1 : 3 * gr.act.max_passes + 4; }
+int tile_launches(const Group& gr) { return gr.act.tile && gr.act.max_n > kSmallBuildN ? 1 + 3 * tile_passes(gr.d) : 0; }
 int group_launches(const Group& gr) { return 1 + sort_launches(gr) + tile_launches(gr) + 2 + 1 + 1 + 3; }
 
 // Kernels of the loop graph: gate and control every iteration, and each
@@ -1007,7 +1012,7 @@ int run_batch(egg_batch_item* items, int count, const egg_opts* opts_in, egg_bat
         const Exec ex = batched(gr.all, gr.d);
         launch_build(ex, S.st);
         launch_labels_uf(ex, S.st);
-        launches += 3 * gr.all.max_passes + 6 + 4;
+        launches += sort_launches(gr) + 2 + 4;
     }
     k_batch_results<<<(count + 255) / 256, 256, 0, S.st>>>(P.d_works, count, P.d_results);
     launches++;

@@ -34,6 +34,13 @@ enum : int {
     kErrStencil = 4,
 };
 
+// Sets of at most this many points are sorted and indexed by one cluster of
+// thread blocks (k_build_small): its phases are cluster barriers apart instead
+// of launches.  The line: a run's first ten iterations, per-pass launches
+// against the cluster, take 11.1 and 10.7 ms at 100,000 x 4 and 9.2 and 8.6 ms
+// at 131,072 x 3, but 15.9 and 17.7 ms at 250,000 x 3, where 16 SMs are too few.
+constexpr int kSmallBuildN = 131072;
+
 // The update kernel's point-by-point walks read a candidate point's
 // coordinates and its sin / 1 - cos offsets as whole 16-byte records when
 // packed_dims(d): pack_w(d) float4 of coordinates, pack_s(d) float4 of the
@@ -106,6 +113,7 @@ struct Work {
     int* perm_tmp;     // [ns]
     unsigned* skey[2]; // [ns] each: whole 32-bit sort keys of the one-key grid sort (d <= 3 and at most
                        // 256 cells per dimension; nullptr otherwise: the per-dimension passes)
+    unsigned* bkey;    // [words][ns] packed sort keys of k_build_small (n <= kSmallBuildN; else nullptr)
     int* cell_of;      // [ns]   cell index of sorted point i
     // cells (index < M, M only known on the device)
     int* cell_start;   // [ns+1]
@@ -325,6 +333,17 @@ template <int D>
 __device__ __forceinline__ float* group_rec(const Work& w, int warp, int rec, int d) {
     return w.gpart + ((size_t)warp * 2 + rec) * group_w(D > 0 ? D : d);
 }
+
+// The packed sort key of a point: the sub-cell digit in the low bits, then the
+// cell coordinates in the order of the per-dimension passes (plan_pass), each
+// in as many bits as the grid's width needs.
+__host__ __device__ inline int key_sub_bits(const Geom& g) { return g.sub_dims * g.sub_bits; }
+__host__ __device__ inline int key_dim_bits(const Geom& g) {
+    int b = 1;
+    while ((g.width - 1) >> b) b++;
+    return b;
+}
+__host__ __device__ inline int key_bits(const Geom& g) { return key_sub_bits(g) + g.d * key_dim_bits(g); }
 
 // cells of this geometry carry byte keys (Work::cell_bytes)
 __host__ __device__ inline bool byte_keys(const Geom& g) { return g.d > 4 && g.d <= kByteDims && g.width <= 256; }

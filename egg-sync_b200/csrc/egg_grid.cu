@@ -19,7 +19,10 @@
 //
 // Every kernel is a device body over its block index (bx, gx) with a
 // single-instance wrapper and a batched wrapper (egg_batch.cuh).
+#include <cooperative_groups.h>
+
 #include "egg_common.cuh"
+#include "egg_host_common.h"
 #include "egg_kernels.h"
 
 namespace egg {
@@ -474,6 +477,41 @@ __device__ __forceinline__ void tile_keys_body(const Geom& g, const Work& w, int
     }
 }
 
+// the records of cell c, whose first sorted point is i and whose coordinate in
+// dimension l is at(l)
+template <int D, typename F>
+__device__ __forceinline__ void write_cell(const Geom& g, const Work& w, int c, int i, F&& at) {
+    const int d = D > 0 ? D : g.d;
+    w.cell_start[c] = i;
+    int outer = 0;
+    unsigned long long key = 0;
+    unsigned b[kByteDims / 4] = {};
+    for (int l = 0; l < d; l++) {
+        const int gl = at(l);
+        w.cell_dims[(size_t)l * g.ns + c] = gl;
+        if (l < g.od) outer += gl * g.wpow[l];
+        if (l < 4) key |= (unsigned long long)gl << (16 * l);
+        if (l < kByteDims) b[l >> 2] |= (unsigned)gl << (8 * (l & 3));
+    }
+    w.cell_outer[c] = outer;
+    if (d <= 4 && w.cell_key) w.cell_key[c] = key;
+    if (w.cell_bytes)
+        *reinterpret_cast<uint4*>(w.cell_bytes + (size_t)c * kByteDims) = make_uint4(b[0], b[1], b[2], b[3]);
+}
+
+// control words of a new grid of M cells (one thread)
+__device__ __forceinline__ void grid_made(const Geom& g, const Work& w, int M) {
+    w.ctrl[kCtrlM] = M;
+    w.ctrl[kCtrlGridValid] = 1;
+    w.ctrl[kCtrlBuilds] += 1;
+    // the tile order goes with the grid; a new one is made where it pays
+    w.ctrl[kCtrlTiled] = 0;
+    w.ctrl[kCtrlTileWant] = tile_order_pays(g, w) ? 1 : 0;
+    // the spanning-cell lists describe the grid: rebuilt with it
+    w.ctrl[kCtrlSpanCount] = 0;
+    w.ctrl[kCtrlBigCount] = 0;
+}
+
 // single-block exclusive scan of the per-block head counts; M = total
 __device__ __forceinline__ void scan_block_sums_body(const Geom& g, const Work& w) {
     EGG_SKIP_IF_UNCHANGED(w.ctrl);
@@ -492,15 +530,7 @@ __device__ __forceinline__ void scan_block_sums_body(const Geom& g, const Work& 
         run += v;
     }
     if (threadIdx.x == 0) {
-        w.ctrl[kCtrlM] = total;
-        w.ctrl[kCtrlGridValid] = 1;
-        w.ctrl[kCtrlBuilds] += 1;
-        // the tile order goes with the grid; a new one is made where it pays
-        w.ctrl[kCtrlTiled] = 0;
-        w.ctrl[kCtrlTileWant] = tile_order_pays(g, w) ? 1 : 0;
-        // the spanning-cell lists describe the grid: rebuilt with it
-        w.ctrl[kCtrlSpanCount] = 0;
-        w.ctrl[kCtrlBigCount] = 0;
+        grid_made(g, w, total);
     }
 }
 
@@ -525,23 +555,7 @@ __device__ __forceinline__ void heads_finalize_body(const Geom& g, const Work& w
         w.cell_of[i] = c;
         w.orig[i] = w.orig_tmp[i];
         if (head) {
-            w.cell_start[c] = i;
-            int outer = 0;
-            unsigned long long key = 0;
-            for (int l = 0; l < d; l++) {
-                int gl = cell_dim(w.X[(size_t)l * g.ns + i], g);
-                w.cell_dims[(size_t)l * g.ns + c] = gl;
-                if (l < g.od) outer += gl * g.wpow[l];
-                if (l < 4) key |= (unsigned long long)gl << (16 * l);
-            }
-            w.cell_outer[c] = outer;
-            if (d <= 4 && w.cell_key) w.cell_key[c] = key;
-            if (w.cell_bytes) {
-                unsigned b[kByteDims / 4] = {};
-                for (int l = 0; l < d; l++)
-                    b[l >> 2] |= (unsigned)cell_dim(w.X[(size_t)l * g.ns + i], g) << (8 * (l & 3));
-                *reinterpret_cast<uint4*>(w.cell_bytes + (size_t)c * kByteDims) = make_uint4(b[0], b[1], b[2], b[3]);
-            }
+            write_cell<D>(g, w, c, i, [&](int l) { return cell_dim(w.X[(size_t)l * g.ns + i], g); });
         }
         if (i == g.n - 1) w.cell_start[c + 1] = g.n;
     }
@@ -574,6 +588,254 @@ __device__ __forceinline__ void outer_ranges_body(const Geom& g, const Work& w, 
                 atomicOr(w.colmask + oc, ((unsigned long long)hi << 32) | lo);
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// The whole build of a small set by one thread-block cluster: the same stable
+// LSD sort (8-bit digits of the packed key, a contiguous run of points per
+// warp), cells and outer ranges.  The build of a small set is 15 to 55
+// launches of 2 to 4 us with next to nothing to do; here the phases are
+// cluster barriers apart, and the blocks exchange digit counts through
+// distributed shared memory.  Bound by the chain of dependent passes (one per
+// key byte, each a counting and a scattering sweep over L2-resident keys).
+// Everything before the update, per run, launches against the cluster: 150 x 4
+// 0.44 and 0.30 ms, 10,000 x 2 0.87 and 0.64 ms, 45,781 x 3 2.85 and 2.15 ms;
+// a whole run of 20,000 x 16 (18 passes) 7.0 and 5.5 ms.
+// ---------------------------------------------------------------------------
+constexpr int kSmallWarps = 16;  // per block
+// Blocks of the cluster: one where a block has next to nothing to do, 16 (more
+// than the portable 8) where the passes take longer than the barriers.  Before
+// the update, per run: 10,000 x 2 0.98, 0.84 and 0.86 ms with 4, 8 and 16
+// blocks; a run of 20,000 x 16 6.4, 5.9 and 5.6 ms.
+inline int small_cluster(int n) { return n <= 1024 ? 1 : (n <= 16384 ? 8 : 16); }
+
+template <int D>
+__device__ __forceinline__ void build_small_body(const Geom& g, const Work& w) {
+    EGG_SKIP_IF_UNCHANGED(w.ctrl);
+    __shared__ int cnt[kSmallWarps][256];
+    __shared__ int base[256];
+    __shared__ int wsum[kSmallWarps];
+    __shared__ int total[256];  // this block's points per digit; total[0] also: its heads
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank_c = (int)cluster.block_rank(), C = (int)cluster.num_blocks();
+    auto barrier = [&]() {
+        if (C > 1) cluster.sync();
+        else __syncthreads();
+    };
+    constexpr int kAhead = 4;  // rounds of 32 points whose loads are in flight together
+    const int d = D > 0 ? D : g.d;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = g.n;
+    const int b = key_dim_bits(g), sb = key_sub_bits(g);
+    const int W = (key_bits(g) + 31) / 32;
+    const int nin = d - g.od;
+    const int len = ((n + C * kSmallWarps - 1) / (C * kSmallWarps) + 31) & ~31;
+    const int i0 = min(n, (rank_c * kSmallWarps + wid) * len), i1 = min(n, i0 + len);
+    const int T = C * 32 * kSmallWarps, gt = rank_c * 32 * kSmallWarps + tid;
+    for (int i = gt; i < n; i += T) {
+        unsigned long long bits = (unsigned)digit_of(g, w.Xn, i, -1, 0);
+        int have = sb, word = 0;
+        for (int k = 0; k < d; k++) {
+            const int l = k < nin ? d - 1 - k : k - nin;  // the order of the per-dimension passes
+            bits |= (unsigned long long)(unsigned)cell_dim(__ldg(w.Xn + (size_t)l * g.ns + i), g) << have;
+            have += b;
+            if (have >= 32) {
+                w.bkey[(size_t)word++ * g.ns + i] = (unsigned)bits;
+                bits >>= 32;
+                have -= 32;
+            }
+        }
+        if (word < W) w.bkey[(size_t)word * g.ns + i] = (unsigned)bits;
+    }
+    barrier();
+    // the stable sort of the packed keys: the permutation ends in perm
+    auto sort = [&](int P) {
+        for (int p = 0; p < P; p++) {
+            const unsigned* kw = w.bkey + (size_t)(p >> 2) * g.ns;
+            const int sh = 8 * (p & 3);
+            // ping-pong that ends in perm
+            const int* in = ((P - p) & 1) ? w.perm_tmp : w.perm;
+            int* out = ((P - 1 - p) & 1) ? w.perm_tmp : w.perm;
+            for (int t = lane; t < 256; t += 32) cnt[wid][t] = 0;
+            __syncwarp();
+            for (int r0 = i0; r0 < i1; r0 += 32 * kAhead) {
+                int dg[kAhead];
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) {
+                    const int i = r0 + 32 * u + lane;
+                    dg[u] = i < i1 ? (int)((kw[p > 0 ? in[i] : i] >> sh) & 255u) : 256 + lane;
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) {
+                    const unsigned peers = __match_any_sync(0xffffffffu, dg[u]);
+                    if (dg[u] < 256 && (peers & lanemask_lt()) == 0) cnt[wid][dg[u]] += __popc(peers);
+                    __syncwarp();
+                }
+            }
+            __syncthreads();
+            if (tid < 256) {
+                int run = 0;
+#pragma unroll
+                for (int q = 0; q < kSmallWarps; q++) {
+                    const int v = cnt[q][tid];
+                    cnt[q][tid] = run;
+                    run += v;
+                }
+                total[tid] = run;
+            }
+            barrier();
+            if (tid < 256) {
+                // the digit's points in all blocks and in those before this one
+                int all = 0, before = 0;
+                for (int q = 0; q < C; q++) {
+                    const int v = cluster.map_shared_rank(total, q)[tid];
+                    if (q < rank_c) before += v;
+                    all += v;
+                }
+                // exclusive scan over the digits: within the warp, then over the eight warps
+                int incl = all;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                if (lane == 31) wsum[wid] = incl;
+                base[tid] = incl - all + before;
+            }
+            __syncthreads();
+            if (tid < 256) {
+                int add = 0;
+                for (int q = 0; q < wid; q++) add += wsum[q];
+                base[tid] += add;
+            }
+            __syncthreads();
+            for (int r0 = i0; r0 < i1; r0 += 32 * kAhead) {
+                int j[kAhead], dg[kAhead];
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) {
+                    const int i = r0 + 32 * u + lane;
+                    j[u] = i < i1 ? (p > 0 ? in[i] : i) : 0;
+                    dg[u] = i < i1 ? (int)((kw[j[u]] >> sh) & 255u) : 256 + lane;
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) {
+                    const unsigned peers = __match_any_sync(0xffffffffu, dg[u]);
+                    const int rank = __popc(peers & lanemask_lt());
+                    int at = 0;
+                    if (dg[u] < 256) at = cnt[wid][dg[u]];
+                    __syncwarp();
+                    if (dg[u] < 256) {
+                        if (rank == 0) cnt[wid][dg[u]] = at + __popc(peers);
+                        out[base[dg[u]] + at + rank] = j[u];
+                    }
+                    __syncwarp();
+                }
+            }
+            barrier();
+        }
+    };
+    sort((key_bits(g) + 7) / 8);
+    // heads: the first sorted points of the cells (the keys' cell bits differ)
+    auto head_of = [&](int i, int j, int jp) {
+        if (i == 0) return true;
+        bool diff = ((w.bkey[j] ^ w.bkey[jp]) >> sb) != 0;
+        for (int k = 1; k < W && !diff; k++) diff = w.bkey[(size_t)k * g.ns + j] != w.bkey[(size_t)k * g.ns + jp];
+        return diff;
+    };
+    int heads = 0;
+    for (int r0 = i0; r0 < i1; r0 += 32) {
+        const int i = r0 + lane;
+        bool head = false;
+        if (i < i1) {
+            const int j = w.perm[i];
+            head = head_of(i, j, i > 0 ? w.perm[i - 1] : 0);
+#pragma unroll 4
+            for (int l = 0; l < d; l++) w.X[(size_t)l * g.ns + i] = __ldg(w.Xn + (size_t)l * g.ns + j);
+            w.orig_tmp[i] = w.orig[j];
+        }
+        heads += __popc(__ballot_sync(0xffffffffu, head));
+    }
+    if (lane == 0) wsum[wid] = heads;
+    if (g.od < d && w.colmask != nullptr)
+        for (int o = gt; o < g.n_outer; o += T) w.colmask[o] = 0ull;
+    __syncthreads();
+    int before = 0, M = 0;
+    for (int k = 0; k < kSmallWarps; k++) {
+        if (k < wid) before += wsum[k];
+        M += wsum[k];
+    }
+    if (tid == 0) total[0] = M;
+    barrier();
+    M = 0;
+    for (int q = 0; q < C; q++) {
+        const int v = cluster.map_shared_rank(total, q)[0];
+        if (q < rank_c) before += v;
+        M += v;
+    }
+    if (gt == 0) grid_made(g, w, M);
+    for (int r0 = i0; r0 < i1; r0 += 32) {
+        const int i = r0 + lane;
+        int j = 0;
+        bool head = false;
+        if (i < i1) {
+            j = w.perm[i];
+            head = head_of(i, j, i > 0 ? w.perm[i - 1] : 0);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, head);
+        if (i < i1) {
+            const int c = before + __popc(m & lanemask_lt()) + (head ? 1 : 0) - 1;
+            w.cell_of[i] = c;
+            w.orig[i] = w.orig_tmp[i];
+            if (head)
+                write_cell<D>(g, w, c, i, [&](int l) {
+                    const int pos = sb + (l >= g.od ? d - 1 - l : nin + l) * b, word = pos >> 5, s = pos & 31;
+                    unsigned long long v = w.bkey[(size_t)word * g.ns + j];
+                    if (s + b > 32) v |= (unsigned long long)w.bkey[(size_t)(word + 1) * g.ns + j] << 32;
+                    return (int)((v >> s) & ((1u << b) - 1u));
+                });
+            if (i == n - 1) w.cell_start[c + 1] = n;
+        }
+        before += __popc(m);
+    }
+    barrier();  // also: no block leaves while another reads its shared memory
+    outer_ranges_body(g, w, rank_c, C);
+    if constexpr (tile_dims(D)) {
+        // the tile order, where the new grid wants one
+        if (!tile_capable(g) || *(volatile int*)(w.ctrl + kCtrlTileWant) == 0) return;
+        const int cut = max(0, 32 - __clz(g.width - 1) - kTileBits);  // cells wider than the key's bits share a code
+        for (int i = gt; i < n; i += T) {
+            const int c = w.cell_of[i];
+            unsigned v[D];
+#pragma unroll
+            for (int l = 0; l < D; l++) v[l] = (unsigned)w.cell_dims[(size_t)l * g.ns + c] >> cut;
+            w.bkey[i] = hilbert_index<D>(v, kTileBits);
+        }
+        if (gt == 0) w.ctrl[kCtrlTileSorts] += 1;
+        barrier();
+        sort(tile_passes(D));
+        if (gt == 0) w.ctrl[kCtrlTiled] = 1;
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * kSmallWarps) k_build_small(Geom g, Work w) {
+    build_small_body<D>(g, w);
+}
+
+// a cluster per active instance
+template <int D>
+__global__ void __launch_bounds__(32 * kSmallWarps) kb_build_small(BatchArgs B) {
+    __shared__ Geom s_g;
+    __shared__ Work s_w;
+    const int k = blockIdx.x / cooperative_groups::this_cluster().num_blocks();
+    if (k >= *B.nact) return;
+    const int inst = B.active[k];
+    const int* sg = reinterpret_cast<const int*>(B.geoms + inst);
+    const int* sw = reinterpret_cast<const int*>(B.works + inst);
+    for (int t = threadIdx.x; t < (int)(sizeof(Geom) / 4); t += blockDim.x) reinterpret_cast<int*>(&s_g)[t] = sg[t];
+    for (int t = threadIdx.x; t < (int)(sizeof(Work) / 4); t += blockDim.x) reinterpret_cast<int*>(&s_w)[t] = sw[t];
+    __syncthreads();
+    build_small_body<D>(s_g, s_w);
 }
 
 // dimension l of a cell's sum and box records
@@ -1127,7 +1389,45 @@ void launch_build(const Exec& ex, cudaStream_t st) {
     launch_build_sort(ex, st);
 }
 
+void launch_build_small(const Exec& ex, cudaStream_t st) {
+    const int C = small_cluster(ex.batch() ? ex.bt->max_n : ex.g->n);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ex.batch() ? C * ex.bt->instances : C);
+    cfg.blockDim = dim3(32 * kSmallWarps);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    auto go = [&](auto one, auto batch) {
+        if (ex.batch()) {
+            if (C > 8) EGG_CHECK(cudaFuncSetAttribute(batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            EGG_CHECK(cudaLaunchKernelEx(&cfg, batch, ex.args(0)));
+        } else {
+            if (C > 8) EGG_CHECK(cudaFuncSetAttribute(one, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            EGG_CHECK(cudaLaunchKernelEx(&cfg, one, *ex.g, *ex.w));
+        }
+    };
+    switch (ex.d) {
+        case 1: go(k_build_small<1>, kb_build_small<1>); break;
+        case 2: go(k_build_small<2>, kb_build_small<2>); break;
+        case 3: go(k_build_small<3>, kb_build_small<3>); break;
+        case 4: go(k_build_small<4>, kb_build_small<4>); break;
+        case 5: go(k_build_small<5>, kb_build_small<5>); break;
+        case 6: go(k_build_small<6>, kb_build_small<6>); break;
+        case 8: go(k_build_small<8>, kb_build_small<8>); break;
+        case 16: go(k_build_small<16>, kb_build_small<16>); break;
+        default: go(k_build_small<0>, kb_build_small<0>); break;
+    }
+}
+
 void launch_build_sort(const Exec& ex, cudaStream_t st) {
+    if (ex.small_build()) {
+        launch_build_small(ex, st);
+        return;
+    }
     if (ex.batch()) {
         for (int p = 0; p < ex.bt->max_passes; p++) {
             kb_radix_hist<<<ex.blocks(kShapeTiles, kSortThreads), kSortThreads, 0, st>>>(ex.args(kShapeTiles), p);
@@ -1167,7 +1467,7 @@ void launch_build_sort(const Exec& ex, cudaStream_t st) {
 // the tile order of a rebuilt grid; every kernel returns at once where the
 // rebuild found it does not pay
 void launch_tile_order(const Exec& ex, cudaStream_t st) {
-    if (!ex.tile) return;
+    if (!ex.tile || ex.small_build()) return;  // a cluster's build makes it
     const int blocks = ex.blocks(kShapeCapN256L, 256), P = tile_passes(ex.d);
     auto keys = [&](auto one, auto batch) {
         if (ex.batch()) batch<<<blocks, 256, 0, st>>>(ex.args(kShapeCapN256L));

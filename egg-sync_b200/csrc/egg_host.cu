@@ -175,6 +175,9 @@ size_t layout_work(const Geom& g, int max_iter, char* base, Work& w, float** xin
     add((void**)&w.skey[0], one_key ? 4 * ns : 0);
     add((void**)&w.skey[1], one_key ? 4 * ns : 0);
     if (!one_key) w.skey[0] = w.skey[1] = nullptr;  // the per-dimension passes
+    const bool small = g.n <= kSmallBuildN;
+    add((void**)&w.bkey, small ? 4 * ns * (size_t)((key_bits(g) + 31) / 32) : 0);
+    if (!small) w.bkey = nullptr;
     add((void**)&w.cell_of, 4 * ns);
     add((void**)&w.cell_start, 4 * (ns + 1));
     add((void**)&w.cell_dims, 4 * d * ns);
@@ -537,7 +540,7 @@ bool ensure_graph(Instance& I) {
         cp.conditional.size = 1;
         e = cudaGraphAddNode(&ifnode, body, &tail, 1, &cp);
         // sort body: [sort, gate] -> IF(the new grid wants a tile order) [tile order]
-        const bool tile = tile_capable(I.g);
+        const bool tile = tile_capable(I.g) && I.w.bkey == nullptr;
         cudaGraph_t sbody = nullptr;
         cudaGraphConditionalHandle ht;
         cudaGraphNode_t stail = nullptr;
@@ -799,19 +802,19 @@ int run(const float* x, int64_t n, int32_t d, float eps, float lam, const egg_op
         }
         // launches: reset + transpose; per iteration: begin, grid check,
         // grid sort (3 per radix pass + 4; with one 32-bit key, 1 + 3 per
-        // pass + 4), 2 cell sums, need, [2 order parameter], update, 3 extra
+        // pass + 4; by one block, 1), 2 cell sums, need, [2 order parameter], update, 3 extra
         // check, end; then the final build (begin, check, sort), labels (1
         // or 4 kernels), [2 cell sums + 2 order parameter], [positions].  In
         // the loop graph two gate kernels run every iteration, the grid sort
         // only in iterations where some point changed cell and the extra
         // check only where the update left the flag at 1.
         const bool onekey = I.w.skey[0] != nullptr && g.d <= 3 && g.width <= 256;
-        const int sort_l = onekey ? 3 * (1 + g.d) + 5 : 3 * plan_count(g) + 4;
+        const int sort_l = I.w.bkey ? 1 : (onekey ? 3 * (1 + g.d) + 5 : 3 * plan_count(g) + 4);
         const int build_l = sort_l + 2;
         const int order_l = (g.order_mode == 2 || g.stop_rule == 1) ? 2 : 0;
         // tile order: keys and 3 kernels per pass; in the loop graph behind a
         // gate of its own in every rebuild
-        const int tile_l = tile_capable(g) ? 1 + 3 * tile_passes(g.d) : 0;
+        const int tile_l = tile_capable(g) && !I.w.bkey ? 1 + 3 * tile_passes(g.d) : 0;
         const int final_l = build_l + (opts.labels_mode == 1 ? 1 : 4) + (g.order_mode == 1 ? 4 : 0) +
                             (opts.positions_out ? 1 : 0);
         long long loop_l = (long long)iters * (sort_l + tile_l + 10 + order_l);

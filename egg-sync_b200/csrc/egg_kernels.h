@@ -26,6 +26,8 @@ struct BatchTables {
     int max_passes = 0;           // radix passes of the instance with the most
     int max_table_k = 0;
     bool tile = false;            // some instance may want a tile order
+    int instances = 0;            // of the group
+    int max_n = 0;                // points of the largest
     bool bytes = false;           // every instance has byte keys (d > 4)
     int occ = 8;                  // persistent blocks per SM of a 256-thread kernel
     int update_threads = 256;     // block size of the update kernel: 128 or 256
@@ -50,6 +52,8 @@ struct Exec {
     BatchArgs args(int shape) const {
         return BatchArgs{bt->geoms, bt->works, bt->boff + (size_t)shape * (bt->cap + 1), bt->active, bt->nact};
     }
+    // every instance's grid is built by a cluster of its own
+    bool small_build() const { return bt ? bt->max_n <= kSmallBuildN : w->bkey != nullptr; }
     int table_k() const { return bt ? bt->max_table_k : g->table_k; }
     int update_threads() const { return bt ? bt->update_threads : 128; }
 };
