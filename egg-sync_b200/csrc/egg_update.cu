@@ -268,12 +268,30 @@ __device__ __forceinline__ void negate_pairs(const float* x, unsigned long long*
 // them) cost a thirty-second of a visit.
 //
 // With the joint box too wide the walk does not pay and returns false before
-// any visit: in storage order (tiled false) as soon as the lanes lie in
-// several columns or spread over dimension od (consecutive points of sparse
-// columns are dozens of cells apart there), in tile order only for more than
-// kUnionCols columns (points of an empty region).
+// any visit: for more than kUnionCols columns (points of an empty region), and
+// in storage order (tiled false) when the lanes lie in several columns or
+// spread over dimension od and more than kSpreadCells cells are around them
+// (consecutive points of sparse columns are dozens of cells apart there).
 // ---------------------------------------------------------------------------
 constexpr int kUnionCols = 1024;
+// Whole rows of columns instead of columns where they hold at most this many
+// cells per column: once the points have gathered, nearly every column of the
+// hundreds around a warp is empty, and finding its few cells took 30 chained
+// loads (update of 1M x 3D, 1,000 iterations: 103 ms by columns, 101 by rows;
+// no difference between 1 and 16 cells per column; before that the window in
+// dimension od leaves a column fewer candidates than its row).
+constexpr int kRowFill = 4;
+// In storage order, lanes in several columns walk together when the rows
+// around them hold at most this many cells; else their points are walked one
+// by one, 15 us for a warp's 32 (68,535 x 2D, 1,000 iterations: update 26.7 ms
+// one by one, 15.1 together; 250k x 3D and 1M x 3D gain nothing from more
+// cells, and with 64 lose 3% and 9%).
+constexpr int kSpreadCells = 256;
+// Points of a block at most (its list), and the blocks of a launch from which
+// on a warp takes several rows in storage order: a full chip of them, five per
+// SM.  1M x 3D, 1,000 iterations, update with 2, 4 and 8 rows: 87, 85, 76 ms.
+constexpr int kListMax = 1024;
+constexpr int kRowBlocks = 148 * 5;
 
 // shared memory of one warp, in 16-byte words: its joint box, 32 cell records (key, first
 // point, points | box | sums), then 32 points (coordinates | sums)
@@ -420,6 +438,7 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
     ulonglong2* const cells = sh + box_words(D);
     ulonglong2* const stage = cells + 32 * CW;
     int ncol;
+    bool spread;  // storage order, several columns: only with few candidates in all
     {
         float cols = 1.f, mar = 1.f;
         bool one = true;
@@ -444,7 +463,8 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
                 B.xh[l] = xh;
             }
         }
-        if (tiled ? cols > (float)kUnionCols : !one) return false;
+        if ((tiled || !one) && cols > (float)kUnionCols) return false;
+        spread = !tiled && !one;
         ncol = (int)cols;
         if (lane == 0) {
             const float inv = 1.0f / g.side;
@@ -457,17 +477,43 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
     negate_pairs<D>(x, nx);
     Col<D> col;
     col.sm = col.lg = 0.f;
+    // Whole rows (the columns of one row of dimension 0 follow each other, and
+    // so do their cells) where they hold few cells, column by column otherwise.
+    const int wide0 = od > 0 ? (int)B.wide[0] : 1;
+    const int nrow = od > 1 ? ncol / wide0 : 1;
+    int rowlen = 1;  // columns of a unit
+    if (od > 0 && wide0 > 1) {
+        bool few = true;
+        int held = 0;
+        for (int s0 = 0; s0 < nrow && few; s0 += 32) {
+            int rem = s0 + lane, o = max(0, (int)B.lo[0] - g.r), m = 0;
+#pragma unroll
+            for (int l = 1; l < D; l++)
+                if (l < od) {
+                    const int wide = B.wide[l], q = rem / wide;
+                    o += (max(0, (int)B.lo[l] - g.r) + rem - q * wide) * g.wpow[l];
+                    rem = q;
+                }
+            if (s0 + lane < nrow) m = __ldg(w.outer_begin + o + wide0) - __ldg(w.outer_begin + o);
+            held += __reduce_add_sync(0xffffffffu, m);
+            few = od == D || held <= ncol * kRowFill;
+        }
+        if (few) rowlen = wide0;
+        spread = spread && !(few && held <= kSpreadCells);
+    }
+    if (spread) return false;
+    const int units = rowlen > 1 ? nrow : ncol;
     const int ob = 16 * od;
     const unsigned long long outer = ob >= 64 ? ~0ull : (1ull << ob) - 1ull;  // a packed key's outer coordinates
-    for (int s0 = 0; s0 < ncol; s0 += 32) {
-        // a column per lane: its candidate cells [cb, ce)
+    for (int s0 = 0; s0 < units; s0 += 32) {
+        // a column or a row per lane: its candidate cells [cb, ce)
         int cb = 0, ce = 0;
         {
-            int rem = s0 + lane, o = 0;
-            float exc = rem < ncol ? 0.f : INFINITY;
+            int rem = s0 + lane, o = rowlen > 1 ? max(0, (int)B.lo[0] - g.r) : 0;
+            float exc = rem < units ? 0.f : INFINITY;
 #pragma unroll
             for (int l = 0; l < D; l++)
-                if (l < od) {
+                if (l < od && (l > 0 || rowlen == 1)) {
                     const int wide = B.wide[l], lo = B.lo[l];
                     const int q = rem / wide;
                     const int v = max(0, lo - g.r) + rem - q * wide;
@@ -479,15 +525,15 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
                 }
             if (exc <= B.r2) {
                 cb = __ldg(w.outer_begin + o);
-                ce = __ldg(w.outer_begin + o + 1);
-                if (cb < ce && od < D) {
+                ce = __ldg(w.outer_begin + o + rowlen);
+                if (cb < ce && od < D && rowlen == 1) {
                     const int* keys = w.cell_dims + (size_t)od * g.ns;
                     cb = lower_bound_i(keys, cb, ce, B.lo[od < D ? od : 0] - g.r - 1);
                     ce = lower_bound_i(keys, cb, ce, B.hi[od < D ? od : 0] + g.r + 2);
                 }
             }
         }
-        // the chunk's candidates numbered through, column by column
+        // the chunk's candidates numbered through, unit by unit
         int upto = ce - cb;
 #pragma unroll
         for (int k = 1; k < 32; k <<= 1) {
@@ -600,8 +646,9 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
 
 // One thread per point.  In tile order a warp's points are neighbours in
 // space; otherwise they are 32 in a row of the storage order, the block's
-// warps taking rows from all over it (the points that still move late in a
-// run sit together, and a block shares them out).  A warp none of whose
+// warps taking rows (several of them in a large set) from all over it (the
+// points that still move late in a run sit together, and a block shares them
+// out).  A warp none of whose
 // points is touched keeps them all; one whose points are close enough walks
 // their joint candidates in lockstep; the points of any other go on the
 // block's list, and its warps take them one at a time (walk_point).  Every
@@ -611,32 +658,67 @@ template <int D, int OD>
 __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* __restrict__ counts, int bx, int gx) {
     constexpr int d = D;
     extern __shared__ float4 s_tab[];  // sin, cos, 1 - cos of k * side; then each warp's area
-    __shared__ int s_list[256];
+    __shared__ int s_list[kListMax];
     __shared__ int s_count;
     const int K = g.table_k, TW = 2 * K + 1;
     const int lane = threadIdx.x & 31;
     const bool tiled = tile_dims(D) && w.ctrl[kCtrlTiled] != 0;
-    const int t0 = tiled ? bx * blockDim.x + threadIdx.x : (((int)(threadIdx.x >> 5) * gx + bx) << 5) + lane;
-    const bool valid = t0 < g.n;
-    const int tv = valid ? t0 : g.n - 1;  // lanes past n shadow the last point; their results are dropped
-    const int i = tiled ? w.perm[tv] : tv;
-    // the point and its warp's last violation bits are loaded before the
-    // table's barrier, so their latency overlaps it (most warps late in a
-    // run need nothing else)
-    float x[D];
+    const int it = w.ctrl[kCtrlIter];
+    // rows of 32 points per warp, and the blocks that takes (the others have none)
+    const int rows = tiled ? 1 : min(kListMax / (int)blockDim.x, (gx + kRowBlocks - 1) / kRowBlocks), gxa = (gx + rows - 1) / rows;
+    if (bx >= gxa) return;
+    const int row0 = tiled ? bx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5) : (int)(threadIdx.x >> 5) * rows * gxa + bx;
+    // Rows none of whose points is touched are settled first, several at a
+    // time: their loads overlap each other and the table's barrier (late in a
+    // run nearly all of them).
+    bool viol = false;
+    unsigned heavy = 1u;
+    if (!tiled && w.ctrl[kCtrlChanged] == 0 && counts == nullptr && w.ctrl[kCtrlForce] == 0) {
+        heavy = 0;
+#pragma unroll 4
+        for (int k = 0; k < rows; k++) {
+            const int i = ((row0 + k * gxa) << 5) + lane;
+            const bool valid = i < g.n;
+            int o = 0, z = 0;
+            unsigned wv = 0;
+            if (valid) {
+                wv = w.warp_viol[i >> 5];
 #pragma unroll
-    for (int l = 0; l < d; l++) x[l] = w.X[(size_t)l * g.ns + i];
-    const unsigned wv_last = tiled ? 0u : w.warp_viol[i >> 5];
+                for (int l = 0; l < d; l++) {
+                    const int c = cell_dim(w.X[(size_t)l * g.ns + i], g);
+                    if (l < g.od) o += c * g.wpow[l];
+                    if (l == g.od) z = c / g.zblk;
+                }
+            }
+            const bool need = valid && ((w.need[o] >> z) & 1ull) != 0;
+            if (__any_sync(0xffffffffu, need)) {
+                heavy |= 1u << k;
+            } else {
+                viol |= wv != 0;
+                if (lane == 0 && valid) w.warp_moved[i >> 5] = 0;
+            }
+        }
+    } else if (rows > 1) {
+        heavy = (1u << rows) - 1u;
+    }
     for (int t = threadIdx.x; t < TW; t += blockDim.x)
         s_tab[t] = make_float4(w.table[t], w.table[TW + t], w.table[2 * TW + t], 0.f);
-    const int it = w.ctrl[kCtrlIter];
     if (threadIdx.x == 0) {
         s_count = 0;
         if (bx == 0) w.stamps[4 * it + 1] = globaltimer();
     }
     __syncthreads();
-    bool viol = false;
-    if ((t0 & ~31) < g.n) {  // uniform across the warp
+#pragma unroll 1
+    for (; heavy; heavy &= heavy - 1) {
+        const int t0 = ((row0 + (__ffs(heavy) - 1) * gxa) << 5) + lane;
+        if ((t0 & ~31) >= g.n) break;  // uniform across the warp
+        const bool valid = t0 < g.n;
+        const int tv = valid ? t0 : g.n - 1;  // lanes past n shadow the last point; their results are dropped
+        const int i = tiled ? w.perm[tv] : tv;
+        float x[D];
+#pragma unroll
+        for (int l = 0; l < d; l++) x[l] = w.X[(size_t)l * g.ns + i];
+        const unsigned wv_last = tiled ? 0u : w.warp_viol[i >> 5];
         bool bad = false;  // the point violates
         int gi[D];
         int obase = 0;
