@@ -284,14 +284,22 @@ constexpr int kRowFill = 4;
 // In storage order, lanes in several columns walk together when the rows
 // around them hold at most this many cells; else their points are walked one
 // by one, 15 us for a warp's 32 (68,535 x 2D, 1,000 iterations: update 26.7 ms
-// one by one, 15.1 together; 250k x 3D and 1M x 3D gain nothing from more
+// one by one, 15 together; 250k x 3D and 1M x 3D gain nothing from more
 // cells, and with 64 lose 3% and 9%).
 constexpr int kSpreadCells = 256;
 // Points of a block at most (its list), and the blocks of a launch from which
 // on a warp takes several rows in storage order: a full chip of them, five per
 // SM.  1M x 3D, 1,000 iterations, update with 2, 4 and 8 rows: 87, 85, 76 ms.
+// A batch's blocks go through its points by themselves (one row: 6 x 8 sweep
+// 101.0 ms, rows by this rule 102.7).
 constexpr int kListMax = 1024;
+// Lanes of one place (a column, and near each other in dimension od) that are
+// at least this many walk together when the whole warp does not (68,535 x 2D,
+// eps 0.01, 417 iterations: update 10.2 ms without groups, 7.7 with groups of
+// four and more, 8.2 with any).
+constexpr int kGroupMin = 4;
 constexpr int kRowBlocks = 148 * 5;
+constexpr int kRowsAhead = 4;  // rows whose loads are in flight together
 
 // shared memory of one warp, in 16-byte words: its joint box, 32 cell records (key, first
 // point, points | box | sums), then 32 points (coordinates | sums)
@@ -427,10 +435,9 @@ struct WarpBox {
     float mar, r2;
 };
 
-template <int D, int OD>
+template <int D, int OD, bool tiled>
 __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const float* x, const int* gi, bool act,
-                                           bool tiled, Acc<D>& a, const float4* tab, int K, ulonglong2* sh,
-                                           int lane) {
+                                           Acc<D>& a, const float4* tab, int K, ulonglong2* sh, int lane) {
     constexpr int PW = pack_w(D), PS = pack_s(D), CW = cell_words(D);
     const int od = OD > 0 ? OD : g.od;
     static_assert(sizeof(WarpBox<D>) <= 16 * box_words(D), "the joint box's words");
@@ -648,24 +655,24 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
 // space; otherwise they are 32 in a row of the storage order, the block's
 // warps taking rows (several of them in a large set) from all over it (the
 // points that still move late in a run sit together, and a block shares them
-// out).  A warp none of whose
-// points is touched keeps them all; one whose points are close enough walks
-// their joint candidates in lockstep; the points of any other go on the
-// block's list, and its warps take them one at a time (walk_point).  Every
+// out).  A warp none of whose points is touched keeps them all; one whose
+// points are close enough walks their joint candidates in lockstep; of any
+// other, in storage order, the groups of one place do so each, and the points
+// left go on the block's list, whose warps take them one at a time
+// (walk_point).  Every
 // path visits a superset of the cells the reference visits and applies the
 // reference's per-point box test to each, in the same order.
-template <int D, int OD>
-__device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* __restrict__ counts, int bx, int gx) {
+template <int D, int OD, bool tiled>
+__device__ __forceinline__ void update_rows(const Geom& g, const Work& w, int* __restrict__ counts, int bx, int gx,
+                                            int max_rows, float4* s_tab, int* s_list, int& s_count, volatile unsigned* state) {
     constexpr int d = D;
-    extern __shared__ float4 s_tab[];  // sin, cos, 1 - cos of k * side; then each warp's area
-    __shared__ int s_list[kListMax];
-    __shared__ int s_count;
+    // what a warp keeps across its walks waits in shared memory: the walk wants the registers
+    volatile unsigned &s_heavy = state[0], &s_left = state[1], &s_grp = state[2], &s_listed = state[3];
     const int K = g.table_k, TW = 2 * K + 1;
     const int lane = threadIdx.x & 31;
-    const bool tiled = tile_dims(D) && w.ctrl[kCtrlTiled] != 0;
     const int it = w.ctrl[kCtrlIter];
     // rows of 32 points per warp, and the blocks that takes (the others have none)
-    const int rows = tiled ? 1 : min(kListMax / (int)blockDim.x, (gx + kRowBlocks - 1) / kRowBlocks), gxa = (gx + rows - 1) / rows;
+    const int rows = tiled ? 1 : min(max_rows, (gx + kRowBlocks - 1) / kRowBlocks), gxa = (gx + rows - 1) / rows;
     if (bx >= gxa) return;
     const int row0 = tiled ? bx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5) : (int)(threadIdx.x >> 5) * rows * gxa + bx;
     // Rows none of whose points is touched are settled first, several at a
@@ -675,27 +682,43 @@ __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* _
     unsigned heavy = 1u;
     if (!tiled && w.ctrl[kCtrlChanged] == 0 && counts == nullptr && w.ctrl[kCtrlForce] == 0) {
         heavy = 0;
-#pragma unroll 4
-        for (int k = 0; k < rows; k++) {
-            const int i = ((row0 + k * gxa) << 5) + lane;
-            const bool valid = i < g.n;
-            int o = 0, z = 0;
-            unsigned wv = 0;
-            if (valid) {
-                wv = w.warp_viol[i >> 5];
+        for (int k0 = 0; k0 < rows; k0 += kRowsAhead) {
+            float xs[kRowsAhead][D];
+            unsigned wv[kRowsAhead];
+            unsigned long long nb[kRowsAhead];
 #pragma unroll
-                for (int l = 0; l < d; l++) {
-                    const int c = cell_dim(w.X[(size_t)l * g.ns + i], g);
-                    if (l < g.od) o += c * g.wpow[l];
-                    if (l == g.od) z = c / g.zblk;
+            for (int k = 0; k < kRowsAhead; k++) {
+                const int i = ((row0 + (k0 + k) * gxa) << 5) + lane;
+                if (k0 + k < rows && i < g.n) {
+                    wv[k] = w.warp_viol[i >> 5];
+#pragma unroll
+                    for (int l = 0; l < d; l++) xs[k][l] = w.X[(size_t)l * g.ns + i];
                 }
             }
-            const bool need = valid && ((w.need[o] >> z) & 1ull) != 0;
-            if (__any_sync(0xffffffffu, need)) {
-                heavy |= 1u << k;
-            } else {
-                viol |= wv != 0;
-                if (lane == 0 && valid) w.warp_moved[i >> 5] = 0;
+#pragma unroll
+            for (int k = 0; k < kRowsAhead; k++) {
+                const int i = ((row0 + (k0 + k) * gxa) << 5) + lane;
+                nb[k] = 0;
+                if (k0 + k < rows && i < g.n) {
+                    int o = 0, z = 0;
+#pragma unroll
+                    for (int l = 0; l < d; l++) {
+                        const int c = cell_dim(xs[k][l], g);
+                        if (l < g.od) o += c * g.wpow[l];
+                        if (l == g.od) z = c / g.zblk;
+                    }
+                    nb[k] = (w.need[o] >> z) & 1ull;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kRowsAhead; k++) {
+                const int i = ((row0 + (k0 + k) * gxa) << 5) + lane;
+                if (__any_sync(0xffffffffu, nb[k] != 0)) {
+                    heavy |= 1u << (k0 + k);
+                } else if (k0 + k < rows && i < g.n) {
+                    viol |= wv[k] != 0;
+                    if (lane == 0) w.warp_moved[i >> 5] = 0;
+                }
             }
         }
     } else if (rows > 1) {
@@ -708,9 +731,17 @@ __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* _
         if (bx == 0) w.stamps[4 * it + 1] = globaltimer();
     }
     __syncthreads();
+    if (!tiled && lane == 0) s_heavy = heavy;
+    __syncwarp();
 #pragma unroll 1
-    for (; heavy; heavy &= heavy - 1) {
-        const int t0 = ((row0 + (__ffs(heavy) - 1) * gxa) << 5) + lane;
+    while (true) {
+        if constexpr (!tiled) {
+            heavy = s_heavy;
+            if (heavy == 0) break;
+            __syncwarp();
+            if (lane == 0) s_heavy = heavy & (heavy - 1);
+        }
+        const int t0 = ((row0 + (tiled ? 0 : (__ffs(heavy) - 1) * gxa)) << 5) + lane;
         if ((t0 & ~31) >= g.n) break;  // uniform across the warp
         const bool valid = t0 < g.n;
         const int tv = valid ? t0 : g.n - 1;  // lanes past n shadow the last point; their results are dropped
@@ -718,7 +749,6 @@ __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* _
         float x[D];
 #pragma unroll
         for (int l = 0; l < d; l++) x[l] = w.X[(size_t)l * g.ns + i];
-        const unsigned wv_last = tiled ? 0u : w.warp_viol[i >> 5];
         bool bad = false;  // the point violates
         int gi[D];
         int obase = 0;
@@ -751,19 +781,71 @@ __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* _
         for (int k = 0; k < kUStats; k++) a.st[k] = 0;
         const long long t_walk0 = clock64();
 #endif
-        bool done = false;  // the lanes that need it have their sums (uniform across the warp)
+        bool done = false;    // the point has its sums
+        unsigned listed = 0;  // the lanes whose points go on the list
         if (nm) {
             if (lane == 0) atomicAdd(w.ctrl + kCtrlComputed, __popc(nm));
             ulonglong2* sh = reinterpret_cast<ulonglong2*>(s_tab + TW) + (threadIdx.x >> 5) * warp_words(D);
-            done = walk_union<D, OD>(g, w, x, gi, needs(), tiled, a, s_tab, K, sh, lane);
-            if (!done && needs()) s_list[atomicAdd(&s_count, 1)] = i;
+            if constexpr (tiled) {
+                done = walk_union<D, OD, true>(g, w, x, gi, needs(), a, s_tab, K, sh, lane);
+                if (!done) listed = nm;
+            } else {
+                // all together, or (storage order) by groups of one place
+                if (lane == 0) {
+                    s_left = s_grp = nm;
+                    s_listed = 0;
+                }
+                __syncwarp();
+                bool whole = true;
+#pragma unroll 1
+                while (true) {
+                    const bool mine = (s_grp >> lane) & 1u;
+                    const bool walked = walk_union<D, OD, false>(g, w, x, gi, mine, a, s_tab, K, sh, lane);
+                    done = done || (walked && mine);
+                    unsigned left = s_left, more = 0;
+                    if (walked) left &= ~s_grp;
+                    if (walked || whole) {
+                        while (left) {  // the next group worth a walk
+                            const int first = __ffs(left) - 1;
+                            bool same = (left >> lane) & 1u;
+#pragma unroll
+                            for (int l = 0; l < D; l++) {
+                                const int gf = __shfl_sync(0xffffffffu, gi[l], first);
+                                same = same && abs(gi[l] - gf) <= (l < g.od ? 0 : l == g.od ? kLockZSpan / 2 : g.width);
+                            }
+                            const unsigned grp = __ballot_sync(0xffffffffu, same);
+                            if (__popc(grp) >= kGroupMin) {
+                                more = grp;
+                                break;
+                            }
+                            left &= ~grp;
+                            listed |= grp;
+                        }
+                    } else {
+                        listed |= left;
+                        left = 0;
+                    }
+                    listed |= s_listed;
+                    __syncwarp();
+                    if (lane == 0) {
+                        s_left = left;
+                        s_grp = more;
+                        s_listed = listed;
+                    }
+                    __syncwarp();
+                    whole = false;
+                    if (more == 0) break;
+                }
+                listed = s_listed;
+            }
+            if ((listed >> lane) & 1u) s_list[atomicAdd(&s_count, 1)] = i;
         }
 #ifdef EGG_UPDATE_STATS
         if (nm) {
             const long long dt = clock64() - t_walk0;
             const long long warp_dt = __reduce_max_sync(0xffffffffu, (unsigned)min(dt, 0x7fffffffLL));
-            if (lane == 0) a.st[done ? kUsCyclesShared : kUsCyclesLane] += (unsigned)warp_dt;
-            if (lane == 0 && !done) a.st[kUsLaneWarps] = 1;
+            if (lane == 0) a.st[listed ? kUsCyclesLane : kUsCyclesShared] += (unsigned)warp_dt;
+            if (lane == 0 && listed) a.st[kUsLaneWarps] = 1;
         }
 #endif
         bool moved = false;
@@ -774,7 +856,7 @@ __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* _
             // are not kept up: then the violation bit goes by original index.
             if (w.ctrl[kCtrlChanged] != 0)
                 for (int l = 0; l < d; l++) w.Xn[(size_t)l * g.ns + i] = x[l];
-            bad = tiled || w.ctrl[kCtrlChanged] != 0 ? w.viol_orig[w.orig[i]] != 0 : ((wv_last >> lane) & 1u) != 0;
+            bad = tiled || w.ctrl[kCtrlChanged] != 0 ? w.viol_orig[w.orig[i]] != 0 : ((w.warp_viol[i >> 5] >> lane) & 1u) != 0;
         } else if (valid && done) {
             const int N = a.N;
             const float fN = (float)N;
@@ -835,6 +917,7 @@ __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* _
             if (lane == 0 && v) atomicAdd(w.ustats + k, v);
         }
 #endif
+        if (tiled) break;
     }
     __syncthreads();
     const int todo = s_count;
@@ -848,14 +931,33 @@ __device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* _
     }
 }
 
+// The two orders are compiled apart: one body for both cost the first
+// iterations (tile order) 3% to 17%.
+template <int D, int OD>
+__device__ __forceinline__ void update_body(const Geom& g, const Work& w, int* __restrict__ counts, int bx, int gx,
+                                            int max_rows) {
+    extern __shared__ float4 s_tab[];  // sin, cos, 1 - cos of k * side; then each warp's area
+    __shared__ int s_list[kListMax];
+    __shared__ int s_count;
+    __shared__ volatile unsigned s_state[8][4];
+    volatile unsigned* const state = s_state[threadIdx.x >> 5];
+    if constexpr (tile_dims(D)) {
+        if (w.ctrl[kCtrlTiled] != 0) {
+            update_rows<D, OD, true>(g, w, counts, bx, gx, max_rows, s_tab, s_list, s_count, state);
+            return;
+        }
+    }
+    update_rows<D, OD, false>(g, w, counts, bx, gx, max_rows, s_tab, s_list, s_count, state);
+}
+
 template <int D, int OD>
 __global__ void __launch_bounds__(128, update_min_blocks(D, 128)) k_update(Geom g, Work w, int* __restrict__ counts) {
-    update_body<D, OD>(g, w, counts, blockIdx.x, gridDim.x);
+    update_body<D, OD>(g, w, counts, blockIdx.x, gridDim.x, kListMax / 128);
 }
 
 template <int D, int T>
 __global__ void __launch_bounds__(T, update_min_blocks(D, T)) kb_update(BatchArgs B) {
-    batch_for(B, [&](const Geom& g, const Work& w, int bx, int gx) { update_body<D, 0>(g, w, nullptr, bx, gx); });
+    batch_for(B, [&](const Geom& g, const Work& w, int bx, int gx) { update_body<D, 0>(g, w, nullptr, bx, gx, 1); });
 }
 
 // need[] (zeroed by the grid-build check of this iteration) receives, over
