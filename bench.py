@@ -429,7 +429,10 @@ def cpu_baseline(X, eps, sample, full_c1=True):
     from eggsync import data
     from oracle import RefSync
 
-    R = RefSync()
+    try:
+        R = RefSync()
+    except FileNotFoundError as e:
+        return {"unavailable": "the reference's CPU SynC is not built here (%s)" % Path(str(e)).name}
     n = len(X)
     per_iter, dt = cpu_iteration_time(R, X, eps, sample)
     out = {
