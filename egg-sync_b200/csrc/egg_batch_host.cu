@@ -415,8 +415,7 @@ void set_tables(Plan& P, const Config& c) {
             bt->update_threads = c.update_threads;
             bt->max_passes = 0;
             bt->max_table_k = 0;
-            bt->tile = false;
-            bt->bytes = true;
+            bt->tile = bt->key8 = bt->key16 = false;
             bt->instances = bt->max_n = 0;
             for (int s = 0; s < kShapeCount; s++) bt->total[s] = 0;
             for (int i = 0; i < P.count; i++) {
@@ -424,9 +423,9 @@ void set_tables(Plan& P, const Config& c) {
                 bt->max_passes = std::max(bt->max_passes, plan_count(P.geoms[i]));
                 bt->max_table_k = std::max(bt->max_table_k, P.geoms[i].table_k);
                 bt->tile = bt->tile || tile_capable(P.geoms[i]);
+                (byte_keys(P.geoms[i]) ? bt->key8 : bt->key16) = true;
                 bt->instances++;
                 bt->max_n = std::max(bt->max_n, P.geoms[i].n);
-                bt->bytes = bt->bytes && byte_keys(P.geoms[i]);
                 for (int s = 0; s < kShapeCount; s++) bt->total[s] += shape_blocks(s, P.geoms[i]);
             }
         }
@@ -490,7 +489,8 @@ std::vector<char> graph_key(const Plan& P) {
         put(&g.act.max_passes, sizeof(int));
         put(&g.act.max_table_k, sizeof(int));
         put(&g.act.tile, sizeof(bool));
-        put(&g.act.bytes, sizeof(bool));
+        put(&g.act.key8, sizeof(bool));
+        put(&g.act.key16, sizeof(bool));
         put(&g.act.instances, sizeof(int));
         put(&g.act.max_n, sizeof(int));
     }
@@ -850,7 +850,8 @@ int enqueue_prologue(State& S, Plan& P, int max_iter) {
 // tables), tile order (keys, 3 per pass), cell sums (2), need, update, extra check (3)
 int sort_launches(const Group& gr) { return gr.act.max_n <= kSmallBuildN ? 1 : 3 * gr.act.max_passes + 4; }
 int tile_launches(const Group& gr) { return gr.act.tile && gr.act.max_n > kSmallBuildN ? 1 + 3 * tile_passes(gr.d) : 0; }
-int group_launches(const Group& gr) { return 1 + sort_launches(gr) + tile_launches(gr) + 2 + 1 + 1 + 3; }
+int update_launches(const Group& gr) { return gr.d > 8 && gr.d <= kKeyDims && gr.act.key8 && gr.act.key16 ? 2 : 1; }
+int group_launches(const Group& gr) { return 1 + sort_launches(gr) + tile_launches(gr) + 2 + 1 + update_launches(gr) + 3; }
 
 // Kernels of the loop graph: gate and control every iteration, and each
 // group's kernels in the iterations where it had active instances (the

@@ -61,7 +61,7 @@ __host__ __device__ constexpr int pack_s(int d) { return (2 * d + 3) / 4; }
 __host__ __device__ constexpr int sum_w(int d) { return 4 * pack_s(d); }
 __host__ __device__ constexpr int box_w(int d) { return 4 * pack_w(d); }
 __host__ __device__ constexpr int group_w(int d) { return sum_w(d) + 2 * box_w(d); }
-constexpr int kByteDims = 16;  // cells of d in (4, 16] with width <= 256: one byte per dimension, 16 bytes a cell
+constexpr int kKeyDims = 16;  // cells of d in (4, 16] carry a key of their own (wide_key_bytes)
 
 // Per-instance geometry, exactly as the reference computes it
 // (src/algorithms/EGG_SynC.cu:1249-1260, 1430, 563, 779, 1045).
@@ -120,7 +120,7 @@ struct Work {
     int* cell_dims;    // [d][ns]
     unsigned long long* cell_key;  // [ns] the cell's dims packed 16 bits each (d <= 4): one load per box test
     int* cell_outer;   // [ns]
-    unsigned char* cell_bytes;     // [ns][16] the cell's dims as bytes (4 < d <= 16, width <= 256; else nullptr)
+    unsigned char* cell_wkey;      // [ns][wide_key_bytes] the cell's dims, 16 or 8 bits each (4 < d <= 16; else nullptr)
     float* csum;       // [ns][sum_w(d)] per cell: sum sin(delta) [d], sum (1 - cos(delta)) [d]
     float* cbox;       // [ns][2 * box_w(d)] tight bounding box of the cell's points: lower, then upper corner
     int* outer_begin;  // [n_outer + 1]
@@ -345,8 +345,14 @@ __host__ __device__ inline int key_dim_bits(const Geom& g) {
 }
 __host__ __device__ inline int key_bits(const Geom& g) { return key_sub_bits(g) + g.d * key_dim_bits(g); }
 
-// cells of this geometry carry byte keys (Work::cell_bytes)
-__host__ __device__ inline bool byte_keys(const Geom& g) { return g.d > 4 && g.d <= kByteDims && g.width <= 256; }
+// Bytes of a cell's key for 4 < d <= 16: whole 16-byte words, with 16 bits per
+// dimension (a grid has at most 65,535 cells per dimension) where one word holds
+// them (d <= 8) or the grid needs them, 8 bits where that keeps d > 8 to one word.
+__host__ __device__ inline bool byte_keys(const Geom& g) { return g.d > 8 && g.d <= kKeyDims && g.width <= 256; }
+__host__ __device__ inline int wide_key_bytes(const Geom& g) {
+    if (g.d <= 4 || g.d > kKeyDims) return 0;
+    return g.d <= 8 || byte_keys(g) ? 16 : 32;
+}
 
 // the tile order's curve has 8 bits per dimension, an 8-bit sort pass each
 constexpr int kTileBits = 8;

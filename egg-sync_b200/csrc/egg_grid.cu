@@ -485,18 +485,25 @@ __device__ __forceinline__ void write_cell(const Geom& g, const Work& w, int c, 
     w.cell_start[c] = i;
     int outer = 0;
     unsigned long long key = 0;
-    unsigned b[kByteDims / 4] = {};
+    unsigned k8[kKeyDims / 4] = {}, k16[kKeyDims / 2] = {};
     for (int l = 0; l < d; l++) {
         const int gl = at(l);
         w.cell_dims[(size_t)l * g.ns + c] = gl;
         if (l < g.od) outer += gl * g.wpow[l];
         if (l < 4) key |= (unsigned long long)gl << (16 * l);
-        if (l < kByteDims) b[l >> 2] |= (unsigned)gl << (8 * (l & 3));
+        if (l < kKeyDims) {
+            k8[l >> 2] |= (unsigned)gl << (8 * (l & 3));
+            k16[l >> 1] |= (unsigned)gl << (16 * (l & 1));
+        }
     }
     w.cell_outer[c] = outer;
     if (d <= 4 && w.cell_key) w.cell_key[c] = key;
-    if (w.cell_bytes)
-        *reinterpret_cast<uint4*>(w.cell_bytes + (size_t)c * kByteDims) = make_uint4(b[0], b[1], b[2], b[3]);
+    if (w.cell_wkey) {
+        const int bytes = wide_key_bytes(g);
+        uint4* rec = reinterpret_cast<uint4*>(w.cell_wkey + (size_t)c * bytes);
+        rec[0] = byte_keys(g) ? make_uint4(k8[0], k8[1], k8[2], k8[3]) : make_uint4(k16[0], k16[1], k16[2], k16[3]);
+        if (bytes > 16) rec[1] = make_uint4(k16[4], k16[5], k16[6], k16[7]);
+    }
 }
 
 // control words of a new grid of M cells (one thread)

@@ -183,9 +183,9 @@ size_t layout_work(const Geom& g, int max_iter, char* base, Work& w, float** xin
     add((void**)&w.cell_dims, 4 * d * ns);
     add((void**)&w.cell_key, d <= 4 ? 8 * ns : 0);
     add((void**)&w.cell_outer, 4 * ns);
-    const bool bytes = byte_keys(g);
-    add((void**)&w.cell_bytes, bytes ? 16 * ns : 0);
-    if (!bytes) w.cell_bytes = nullptr;
+    const int wkey = wide_key_bytes(g);
+    add((void**)&w.cell_wkey, (size_t)wkey * ns);
+    if (!wkey) w.cell_wkey = nullptr;
     add((void**)&w.csum, 4 * (size_t)sum_w(d) * ns);
     add((void**)&w.cbox, 4 * 2 * (size_t)box_w(d) * ns);
     add((void**)&w.outer_begin, 4 * ((size_t)g.n_outer + 1));

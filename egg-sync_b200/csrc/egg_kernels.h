@@ -28,7 +28,7 @@ struct BatchTables {
     bool tile = false;            // some instance may want a tile order
     int instances = 0;            // of the group
     int max_n = 0;                // points of the largest
-    bool bytes = false;           // every instance has byte keys (d > 4)
+    bool key8 = false, key16 = false;  // d > 8: some instance's cells have keys of 8, of 16 bits a dimension
     int occ = 8;                  // persistent blocks per SM of a 256-thread kernel
     int update_threads = 256;     // block size of the update kernel: 128 or 256
 };

@@ -74,39 +74,38 @@ __host__ __device__ constexpr int walk_floats(int dm) { return 2 * dm * 33 + 2 *
 #endif
 
 // What the walk knows a cell by.  DM: the dimensions the compiler knows the
-// arrays by (up to 4: 16-bit keys; 5 to 16: byte keys; 0: any d, no keys);
-// EX: d == DM exactly.
-template <int DM, bool EX>
+// arrays by (0: any d, no keys); EX: d == DM exactly; KB: bits of a key's
+// coordinate (8 only where DM > 8).
+template <int DM, bool EX, int KB>
 struct CellReader {
     static constexpr int LM = DM > 0 ? DM : kMaxDims;
     static constexpr int U = DM > 0 ? DM : 1;
-    static constexpr int NW = DM <= 8 ? 2 : 4;  // words of a key
+    static constexpr int NW = DM <= 4 ? 2 : (DM > 8 && KB == 16 ? 8 : 4);  // words of a key
 
     static __device__ __forceinline__ void load_key(const Work& w, int c, unsigned* key) {
         if constexpr (DM > 0 && DM <= 4) {
             const unsigned long long v = __ldg(w.cell_key + c);
             key[0] = (unsigned)v;
             key[1] = (unsigned)(v >> 32);
-        } else if constexpr (NW == 2 && DM > 0) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(w.cell_bytes + (size_t)c * kByteDims));
-            key[0] = v.x;
-            key[1] = v.y;
         } else if constexpr (DM > 0) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(w.cell_bytes + (size_t)c * kByteDims));
-            key[0] = v.x;
-            key[1] = v.y;
-            key[2] = v.z;
-            key[3] = v.w;
+#pragma unroll
+            for (int k = 0; k < NW / 4; k++) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(w.cell_wkey + (size_t)c * (4 * NW)) + k);
+                key[4 * k] = v.x;
+                key[4 * k + 1] = v.y;
+                key[4 * k + 2] = v.z;
+                key[4 * k + 3] = v.w;
+            }
         }
     }
     static __device__ __forceinline__ int coord(const Geom& g, const Work& w, const unsigned* key, int c, int l) {
-        if constexpr (DM > 0 && DM <= 4) return (int)((key[l >> 1] >> (16 * (l & 1))) & 0xffffu);
+        if constexpr (DM > 0 && KB == 16) return (int)((key[l >> 1] >> (16 * (l & 1))) & 0xffffu);
         else if constexpr (DM > 0) return (int)((key[l >> 2] >> (8 * (l & 3))) & 255u);
         else return __ldg(w.cell_dims + (size_t)l * g.ns + c);
     }
     // the coordinate as a float: its bits are the low mantissa of 2^23 + cd
     static __device__ __forceinline__ float coord_f(const Geom& g, const Work& w, const unsigned* key, int c, int l) {
-        if constexpr (DM > 0 && DM <= 4)
+        if constexpr (DM > 0 && KB == 16)
             return __uint_as_float(__byte_perm(key[l >> 1], 0x4b000000u, (l & 1) ? 0x7432 : 0x7410)) - 8388608.0f;
         else if constexpr (DM > 0)
             return __uint_as_float(__byte_perm(key[l >> 2], 0x4b000000u, 0x7440 | (l & 3))) - 8388608.0f;
@@ -116,7 +115,7 @@ struct CellReader {
     // the reference's box sums (EGG_SynC.cu:613-630) of cell c for x
     static __device__ __forceinline__ void box_sums(const Geom& g, const Work& w, int d, const float* x, int c,
                                                     float& sm2, float& lg2) {
-        unsigned key[4];
+        unsigned key[NW];
         load_key(w, c, key);
         sm2 = lg2 = 0.f;
 #pragma unroll U
@@ -167,11 +166,11 @@ struct CellReader {
 // sums[0..LM) and sums[LM..2 LM) of the warp's shared area, |N(p)| and the
 // points counted outside fully covered cells into N and partial_in (every
 // lane).  All 32 lanes of the warp call it.
-template <int DM, bool EX>
+template <int DM, bool EX, int KB>
 __device__ __forceinline__ void walk_point(const Geom& g, const Work& w, const float* x, const int* gi, int own,
                                            const float4* tab, float* area, int lane, int& N_out, int& partial_out,
                                            unsigned* st) {
-    using R = CellReader<DM, EX>;
+    using R = CellReader<DM, EX, KB>;
     constexpr int LM = R::LM, U = R::U, SLOTS = (2 * LM + 31) / 32;
     const int d = EX ? DM : g.d;
     const int K = g.table_k;
@@ -288,7 +287,7 @@ __device__ __forceinline__ void walk_point(const Geom& g, const Work& w, const f
             // within the table: the cell passed the box test)
             float* t = terms + __popc(mask & ((1u << lane) - 1u));
             const float mf = (float)cnt;
-            unsigned key[4];
+            unsigned key[R::NW];
             R::load_key(w, c, key);
 #pragma unroll U
             for (int l = 0; l < LM; l++) {
@@ -355,11 +354,11 @@ __device__ __forceinline__ void walk_point(const Geom& g, const Work& w, const f
 // is the warp's shared memory.  words: the storage warps' violation words are
 // in use (they hold a zero for the point).  Returns whether a point violates
 // (every lane of the warp).
-template <int DM, bool EX>
+template <int DM, bool EX, int KB>
 __device__ __forceinline__ bool update_listed_points(const Geom& g, const Work& w, int* __restrict__ counts,
                                                      const float4* tab, float* area, const int* list, int todo,
                                                      bool words) {
-    using R = CellReader<DM, EX>;
+    using R = CellReader<DM, EX, KB>;
     constexpr int LM = R::LM, U = R::U;
     const int d = EX ? DM : g.d;
     const int lane = threadIdx.x & 31;
@@ -382,9 +381,9 @@ __device__ __forceinline__ bool update_listed_points(const Geom& g, const Work& 
         }
         int N, partial_in;
 #ifdef EGG_UPDATE_STATS
-        walk_point<DM, EX>(g, w, x, gi, own, tab, area, lane, N, partial_in, st);
+        walk_point<DM, EX, KB>(g, w, x, gi, own, tab, area, lane, N, partial_in, st);
 #else
-        walk_point<DM, EX>(g, w, x, gi, own, tab, area, lane, N, partial_in, nullptr);
+        walk_point<DM, EX, KB>(g, w, x, gi, own, tab, area, lane, N, partial_in, nullptr);
 #endif
         // the new position: lane l takes dimension l
         const float fN = (float)N;
@@ -481,10 +480,10 @@ __device__ __forceinline__ bool update_listed_points(const Geom& g, const Work& 
 // eight (a sector of every array) taken from all over the storage order,
 // because those that still move sit together: late in a run the few hundred
 // of them spread over as many blocks.
-template <int DM, bool EX>
+template <int DM, bool EX, int KB>
 __device__ __forceinline__ void update_points_body(const Geom& g, const Work& w, int* __restrict__ counts, int per,
                                                    int bx, int gx) {
-    using R = CellReader<DM, EX>;
+    using R = CellReader<DM, EX, KB>;
     constexpr int LM = R::LM;
     const int d = EX ? DM : g.d;
     extern __shared__ float4 s_tab[];  // sin, cos, 1 - cos of k * side; then each warp's area
@@ -519,7 +518,7 @@ __device__ __forceinline__ void update_points_body(const Geom& g, const Work& w,
     __syncthreads();
     const int todo = s_count;
     if (threadIdx.x == 0 && todo) atomicAdd(w.ctrl + kCtrlComputed, todo);
-    any_viol |= update_listed_points<DM, EX>(g, w, counts, s_tab, area, s_list, todo, false);
+    any_viol |= update_listed_points<DM, EX, KB>(g, w, counts, s_tab, area, s_list, todo, false);
     if (__any_sync(0xffffffffu, any_viol) && lane == 0) {
         volatile int* f = w.ctrl + kCtrlFlag;
         if (*f != 0) *f = 0;

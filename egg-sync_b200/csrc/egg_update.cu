@@ -923,7 +923,7 @@ __device__ __forceinline__ void update_rows(const Geom& g, const Work& w, int* _
     const int todo = s_count;
     if (todo) {
         float* area = reinterpret_cast<float*>(s_tab + TW) + (threadIdx.x >> 5) * (4 * warp_words(D));
-        viol |= update_listed_points<D, true>(g, w, counts, s_tab, area, s_list, todo, !tiled);
+        viol |= update_listed_points<D, true, 16>(g, w, counts, s_tab, area, s_list, todo, !tiled);
     }
     if (__any_sync(0xffffffffu, viol) && lane == 0) {
         volatile int* f = w.ctrl + kCtrlFlag;

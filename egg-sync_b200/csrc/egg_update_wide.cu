@@ -19,15 +19,19 @@ namespace egg {
 namespace {
 
 constexpr int kWideThreads = 128;
-template <int DM, bool EX>
+template <int DM, bool EX, int KB>
 __global__ void __launch_bounds__(kWideThreads) k_update_wide(Geom g, Work w, int* __restrict__ counts, int per) {
-    update_points_body<DM, EX>(g, w, counts, per, blockIdx.x, gridDim.x);
+    update_points_body<DM, EX, KB>(g, w, counts, per, blockIdx.x, gridDim.x);
 }
 
-template <int DM, bool EX>
+// A batch's instances of one d > 8 may differ in their keys' width: a launch
+// for each width takes the instances that have it (one kernel for both wants
+// 252 registers at d = 16, where each alone wants 168).
+template <int DM, bool EX, int KB>
 __global__ void __launch_bounds__(kWideThreads) kb_update_wide(BatchArgs B) {
     batch_for(B, [&](const Geom& g, const Work& w, int bx, int gx) {
-        update_points_body<DM, EX>(g, w, nullptr, kWideBatchPer, bx, gx);
+        if (DM > 8 && byte_keys(g) != (KB == 8)) return;
+        update_points_body<DM, EX, KB>(g, w, nullptr, kWideBatchPer, bx, gx);
     });
 }
 
@@ -58,20 +62,33 @@ void launch_update_wide(const Exec& ex, int* counts, cudaStream_t st) {
             one<<<blocks, kWideThreads, smem, st>>>(*ex.g, *ex.w, counts, per);
         }
     };
-    // byte keys need d <= 16 and at most 256 cells per dimension; a batch's
-    // instances of one d may differ in that, so it takes the keys only where
-    // every one has them
-    const bool bytes = ex.batch() ? ex.bt->bytes : ex.w->cell_bytes != nullptr;
-    if (ex.d == 2) go(k_update_wide<2, true>, kb_update_wide<2, true>, 2);
-    else if (ex.d == 3) go(k_update_wide<3, true>, kb_update_wide<3, true>, 3);
-    else if (ex.d == 4) go(k_update_wide<4, true>, kb_update_wide<4, true>, 4);
-    else if (!bytes) go(k_update_wide<0, false>, kb_update_wide<0, false>, kMaxDims);
-    else if (ex.d == 5) go(k_update_wide<5, true>, kb_update_wide<5, true>, 5);
-    else if (ex.d == 6) go(k_update_wide<6, true>, kb_update_wide<6, true>, 6);
-    else if (ex.d == 8) go(k_update_wide<8, true>, kb_update_wide<8, true>, 8);
-    else if (ex.d == 16) go(k_update_wide<16, true>, kb_update_wide<16, true>, 16);
-    else if (ex.d < 8) go(k_update_wide<8, false>, kb_update_wide<8, false>, 8);
-    else go(k_update_wide<16, false>, kb_update_wide<16, false>, 16);
+    // Every grid of 4 < d <= 16 has keys (16 bits a dimension hold any width), so
+    // only more dimensions take the kernel for any d: 64-entry arrays, one load
+    // per coordinate, 70 KB of shared memory per block.  Above 256 cells per
+    // dimension, that kernel against these: a run of 100k x 5 at eps 0.012 98.1
+    // and 29.8 ms, 20k x 8 at 0.02 8.7 and 4.5, 20k x 16 at 0.03 14.3 and 7.0.
+    switch (ex.d) {
+        case 2: go(k_update_wide<2, true, 16>, kb_update_wide<2, true, 16>, 2); return;
+        case 3: go(k_update_wide<3, true, 16>, kb_update_wide<3, true, 16>, 3); return;
+        case 4: go(k_update_wide<4, true, 16>, kb_update_wide<4, true, 16>, 4); return;
+        case 5: go(k_update_wide<5, true, 16>, kb_update_wide<5, true, 16>, 5); return;
+        case 6: go(k_update_wide<6, true, 16>, kb_update_wide<6, true, 16>, 6); return;
+        case 7: go(k_update_wide<8, false, 16>, kb_update_wide<8, false, 16>, 8); return;
+        case 8: go(k_update_wide<8, true, 16>, kb_update_wide<8, true, 16>, 8); return;
+        default: break;
+    }
+    if (ex.d > kKeyDims) {
+        go(k_update_wide<0, false, 16>, kb_update_wide<0, false, 16>, kMaxDims);
+        return;
+    }
+    const bool k8 = ex.batch() ? ex.bt->key8 : byte_keys(*ex.g), k16 = ex.batch() ? ex.bt->key16 : !k8;
+    if (ex.d == 16) {
+        if (k8) go(k_update_wide<16, true, 8>, kb_update_wide<16, true, 8>, 16);
+        if (k16) go(k_update_wide<16, true, 16>, kb_update_wide<16, true, 16>, 16);
+    } else {
+        if (k8) go(k_update_wide<16, false, 8>, kb_update_wide<16, false, 8>, 16);
+        if (k16) go(k_update_wide<16, false, 16>, kb_update_wide<16, false, 16>, 16);
+    }
 }
 
 }  // namespace egg
