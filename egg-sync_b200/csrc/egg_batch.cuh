@@ -17,7 +17,6 @@
 namespace egg {
 
 constexpr int kScanSmallTiles = 64;  // radix digit scan: one block per instance up to this many tiles
-constexpr int kWideBatchPer = 16;    // points per block of the wide update (d > 4) in a batch
 constexpr int kMaxBatch = 1024;      // instances of one batched call
 
 // launch shapes: how many blocks a kernel uses for one instance
@@ -34,7 +33,7 @@ enum Shape : int {
     kShapeCapOuter,    // min(ceil(n_outer / 64), 148 * 8): 8 outer cells per warp
     kShapeFix,         // min(ceil(ceil(n / 32) / 8), 148 * 8)
     kShapeCapN256L,    // min(ceil(n / 256), 148 * 16)
-    kShapeWide,        // ceil(n / kWideBatchPer): kWideBatchPer points a block (d > 4)
+    kShapeWide,        // wide update: wide_per points a block, in whole runs of eight from eight on
     kShapeCount
 };
 
@@ -56,7 +55,7 @@ __host__ __device__ inline int shape_blocks(int shape, const Geom& g) {
         case kShapeCapOuter: return cap(cdiv(g.n_outer, 64) > 0 ? cdiv(g.n_outer, 64) : 1, 148 * 8);
         case kShapeFix: return cap(cdiv(cdiv(g.n, 32), 8), 148 * 8);
         case kShapeCapN256L: return cap(cdiv(g.n, 256), 148 * 16);
-        case kShapeWide: return cdiv(g.n, kWideBatchPer);
+        case kShapeWide: return g.wide_per < 8 ? cdiv(g.n, g.wide_per) : cdiv(cdiv(g.n, 8), g.wide_per / 8);
         default: return 1;
     }
 }
@@ -81,6 +80,26 @@ __host__ __device__ inline void plan_pass(const Geom& g, int p, int& dim, int& s
 }
 
 __host__ __device__ inline int plan_out_sel(int count, int p) { return ((count - p) & 1) ? 0 : 1; }
+
+constexpr int kWideThreads = 128;
+
+// Points per block of the wide update, for `points` of one launch.  Where every
+// point is recomputed each wants a warp (the heavy ones, those of a dense
+// cluster, sit together: 100k x 5D, ten iterations, 15.2 ms with one point per
+// warp against 16.8 with two, 18.6 with four); from some 75,000 warps on, blocks
+// that only settle kept points would be too many.  A batch counts the points of
+// all its instances of a dimension: 200 instances with 4.9M points of five
+// dimensions take 745 ms with 16 points a block and 694 with 128, 16 with
+// 480,000 of eight 79 with 16 and 92 with 128.  Its blocks load descriptors and
+// table again for each instance they meet, so it stays at kWideBatchPer and more
+// (200 instances with 60,000 points of eight dimensions: 3.6 ms with 16, 3.9
+// with 4).
+constexpr int kWideBatchPer = 16;
+inline int wide_points_per_block(long long points) {
+    int per = kWideThreads;
+    while (per > kWideThreads / 32 && (points + per - 1) / per < 148 * 128) per >>= 1;
+    return per;
+}
 
 struct BatchArgs {
     const Geom* geoms;   // [instances]

@@ -705,7 +705,14 @@ void make_plan(State& S, Plan& P, egg_batch_item* items, int count, const egg_op
     for (size_t k = 0; k < ds.size(); k++) {
         P.groups[k].d = ds[k];
         int m = 0;
-        for (int i = 0; i < count; i++) m += P.geoms[i].d == ds[k];
+        long long points = 0;
+        for (const Geom& g : P.geoms)
+            if (g.d == ds[k]) {
+                m++;
+                points += g.n;
+            }
+        for (Geom& g : P.geoms)
+            if (g.d == ds[k]) g.wide_per = std::max(kWideBatchPer, wide_points_per_block(points));
         P.cap = std::max(P.cap, m);
     }
     const size_t ws_bytes = off;
@@ -915,10 +922,11 @@ Config autotune(State& S, Plan& P) {
     time_trial(S, P, best);  // warm-up: graph instantiation, caches
     auto trial2 = [&](const Config& c) { return std::min(time_trial(S, P, c), time_trial(S, P, c)); };
     float tb = trial2(best);
-    // the trials see the first iterations only, where nearly every point is
-    // recomputed; blocks of 256 cost least in the many that follow (one sweep's
-    // last 500 iterations: 36.6 ms, 40 with 128 and 46 with 64), so the others
-    // have to be 5% ahead
+    // The trials see the first iterations only, where nearly every point is
+    // recomputed; what the many that follow want differs from sweep to sweep (48
+    // instances of up to 68,535 points: 69.3 ms with blocks of 256, 72.1 with 128;
+    // 144 two-dimensional ones of up to 179,575: 183 and 175), so another size has
+    // to be 5% ahead in the trials.
     auto consider = [&](Config c) {
         const float t = trial2(c);
         if (t < tb * (c.update_threads != best.update_threads ? 0.95f : 1.0f)) {

@@ -90,6 +90,7 @@ struct Geom {
     int zblk;          // incremental update: cells of dimension od per block (1 block when od == d)
     int tile_min;      // points from which d = 2, 3, 4 may run in tile order
     int point_walk;    // the update gives every point a warp of its own
+    int wide_per;      // ... in blocks that settle this many points (wide_points_per_block)
     int nzb;           // ... number of blocks (<= 64: one bit each)
     int wpow[32];      // width^l for l < od
 };

@@ -101,6 +101,7 @@ Geom make_geom(int64_t n64, int d, float eps) {
     }
     g.tile_min = kTileMinN;
     g.point_walk = d > 4 || (d > 1 && !tile_capable(g));
+    g.wide_per = wide_points_per_block(n);
     g.sub_dims = std::min(d, 8);
     g.sub_bits = std::max(1, 8 / g.sub_dims);
     return g;

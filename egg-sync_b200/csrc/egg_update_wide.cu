@@ -18,49 +18,58 @@ namespace egg {
 
 namespace {
 
-constexpr int kWideThreads = 128;
 template <int DM, bool EX, int KB>
-__global__ void __launch_bounds__(kWideThreads) k_update_wide(Geom g, Work w, int* __restrict__ counts, int per) {
-    update_points_body<DM, EX, KB>(g, w, counts, per, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(kWideThreads) k_update_wide(Geom g, Work w, int* __restrict__ counts) {
+    update_points_body<DM, EX, KB>(g, w, counts, g.wide_per, blockIdx.x, gridDim.x);
+}
+
+// Blocks per SM of the batched kernels: the walk's loads want warps, its arrays
+// want registers.  200 instances with 4.9M points of five dimensions: 694 ms
+// with the five blocks that 96 registers give, 619 with seven (72 registers, a
+// few values spilled), 624 with eight, 716 with ten; 18 with 900,000 of six: 204
+// with four, 177 with seven; 16 with 480,000 of eight: 79.4, 76.7 and 78.9 with
+// four, five and six; eight with 80,000 of twelve: 25.9 with three, 23.2 with
+// five; the others differ by less than the runs.
+constexpr int wide_min_blocks(int dm, bool exact) {
+    return dm == 5 || dm == 6 ? 7 : dm == 8 ? (exact ? 5 : 7) : dm == 16 ? (exact ? 4 : 5) : 5;
 }
 
 // A batch's instances of one d > 8 may differ in their keys' width: a launch
 // for each width takes the instances that have it (one kernel for both wants
 // 252 registers at d = 16, where each alone wants 168).
 template <int DM, bool EX, int KB>
-__global__ void __launch_bounds__(kWideThreads) kb_update_wide(BatchArgs B) {
+__global__ void __launch_bounds__(kWideThreads, wide_min_blocks(DM, EX)) kb_update_wide(BatchArgs B) {
     batch_for(B, [&](const Geom& g, const Work& w, int bx, int gx) {
         if (DM > 8 && byte_keys(g) != (KB == 8)) return;
-        update_points_body<DM, EX, KB>(g, w, nullptr, kWideBatchPer, bx, gx);
+        update_points_body<DM, EX, KB>(g, w, nullptr, g.wide_per, bx, gx);
     });
 }
 
 }  // namespace
 
-// Points per block of one instance.  Where every point is recomputed each
-// wants a warp (the heavy ones, those of a dense cluster, sit together: 100k x
-// 5D, ten iterations, 15.2 ms with one point per warp against 16.8 with two,
-// 18.6 with four); from some 75,000 warps on, blocks that only settle kept
-// points would be too many.
-int wide_points_per_block(int n) {
-    int per = kWideThreads;
-    while (per > kWideThreads / 32 && (n + per - 1) / per < 148 * 128) per >>= 1;
-    return per;
-}
-
 void launch_update_wide(const Exec& ex, int* counts, cudaStream_t st) {
-    auto go = [&](auto one, auto batch, int lm) {
-        const size_t smem = 16 * (2 * (size_t)ex.table_k() + 1) + 4 * (size_t)walk_floats(lm) * (kWideThreads / 32);
-        if (ex.batch()) {
-            if (smem > 36 * 1024) cudaFuncSetAttribute(batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            batch<<<ex.blocks(kShapeWide, kWideThreads), kWideThreads, smem, st>>>(ex.args(kShapeWide));
-        } else {
-            if (smem > 46 * 1024) cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            const int per = wide_points_per_block(ex.g->n);
-            const int runs = per < 8 ? per : 8;  // whole runs of eight points
-            const int blocks = ((ex.g->n + runs - 1) / runs + per / runs - 1) / (per / runs);
-            one<<<blocks, kWideThreads, smem, st>>>(*ex.g, *ex.w, counts, per);
+    const size_t table = 16 * (2 * (size_t)ex.table_k() + 1);
+    auto smem_of = [&](int lm) { return table + 4 * (size_t)walk_floats(lm) * (kWideThreads / 32); };
+    auto one = [&](auto kernel, int lm) {
+        const size_t smem = smem_of(lm);
+        if (smem > 46 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kernel<<<shape_blocks(kShapeWide, *ex.g), kWideThreads, smem, st>>>(*ex.g, *ex.w, counts);
+    };
+    // d <= 4 comes here from single calls only
+    if (ex.d <= 4) {
+        if (ex.d == 2) one(k_update_wide<2, true, 16>, 2);
+        else if (ex.d == 3) one(k_update_wide<3, true, 16>, 3);
+        else one(k_update_wide<4, true, 16>, 4);
+        return;
+    }
+    auto go = [&](auto single, auto batch, int lm) {
+        if (!ex.batch()) {
+            one(single, lm);
+            return;
         }
+        const size_t smem = smem_of(lm);
+        if (smem > 36 * 1024) cudaFuncSetAttribute(batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        batch<<<ex.blocks(kShapeWide, kWideThreads), kWideThreads, smem, st>>>(ex.args(kShapeWide));
     };
     // Every grid of 4 < d <= 16 has keys (16 bits a dimension hold any width), so
     // only more dimensions take the kernel for any d: 64-entry arrays, one load
@@ -68,9 +77,6 @@ void launch_update_wide(const Exec& ex, int* counts, cudaStream_t st) {
     // dimension, that kernel against these: a run of 100k x 5 at eps 0.012 98.1
     // and 29.8 ms, 20k x 8 at 0.02 8.7 and 4.5, 20k x 16 at 0.03 14.3 and 7.0.
     switch (ex.d) {
-        case 2: go(k_update_wide<2, true, 16>, kb_update_wide<2, true, 16>, 2); return;
-        case 3: go(k_update_wide<3, true, 16>, kb_update_wide<3, true, 16>, 3); return;
-        case 4: go(k_update_wide<4, true, 16>, kb_update_wide<4, true, 16>, 4); return;
         case 5: go(k_update_wide<5, true, 16>, kb_update_wide<5, true, 16>, 5); return;
         case 6: go(k_update_wide<6, true, 16>, kb_update_wide<6, true, 16>, 6); return;
         case 7: go(k_update_wide<8, false, 16>, kb_update_wide<8, false, 16>, 8); return;

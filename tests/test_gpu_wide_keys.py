@@ -68,6 +68,17 @@ def test_mixed_batch_equals_single_runs(spec):
         assert np.array_equal(labels, s_labels) and info["iterations"] == s_info["iterations"]
 
 
+def test_batch_with_more_points_a_block():
+    """606,208 points and more of one dimension: 32 a block in the batch, 16 in single calls."""
+    from eggsync import egg_sync, egg_sync_batch
+
+    inst = [(points(k, 325_001, 5), eps) for k, eps in enumerate((0.012, 0.03))]
+    out, _ = egg_sync_batch(inst, max_iter=3, tune="off")
+    for (X, eps), (labels, info) in zip(inst, out):
+        s_labels, s_info = egg_sync(X, eps, max_iter=3)
+        assert np.array_equal(labels, s_labels) and info["iterations"] == s_info["iterations"]
+
+
 def test_one_narrow_eps_does_not_slow_its_batch():
     """An instance with more than 256 cells per dimension costs its batch what
     it costs by itself: it used to take every instance of its dimension to the
