@@ -30,6 +30,7 @@
 #include <climits>
 
 #include "egg_common.cuh"
+#include "egg_host_common.h"
 #include "egg_kernels.h"
 #include "egg_point_walk.cuh"
 #include "egg_stencil.cuh"
@@ -1032,8 +1033,11 @@ void launch_need(const Exec& ex, cudaStream_t st) {
 template <int T>
 void launch_update_batch(const Exec& ex, size_t smem, cudaStream_t st) {
     const int shape = T == 128 ? kShapeN128 : kShapeN256;
-    // at most 36 KB (256 threads) beside the descriptors' static 10 KB: below the 48 KB that need no opt-in
-    auto go = [&](auto kernel) { kernel<<<ex.blocks(shape, T), T, smem, st>>>(ex.args(shape)); };
+    // beside 13 KB of descriptors, list and state: 48 KB together need no opt-in
+    auto go = [&](auto kernel) {
+        if (smem > 32 * 1024) EGG_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<ex.blocks(shape, T), T, smem, st>>>(ex.args(shape));
+    };
     switch (ex.d) {
         case 1: go(kb_update<1, T>); break;
         case 2: go(kb_update<2, T>); break;

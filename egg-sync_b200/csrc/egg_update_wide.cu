@@ -11,6 +11,7 @@
 // 0.71 -> 0.24 ms a run (a thread per point before).  25k instructions per
 // point at 100k x 5D; what is left is their issue and the chains of loads.
 #include "egg_common.cuh"
+#include "egg_host_common.h"
 #include "egg_kernels.h"
 #include "egg_point_walk.cuh"
 
@@ -52,7 +53,7 @@ void launch_update_wide(const Exec& ex, int* counts, cudaStream_t st) {
     auto smem_of = [&](int lm) { return table + 4 * (size_t)walk_floats(lm) * (kWideThreads / 32); };
     auto one = [&](auto kernel, int lm) {
         const size_t smem = smem_of(lm);
-        if (smem > 46 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 46 * 1024) EGG_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kernel<<<shape_blocks(kShapeWide, *ex.g), kWideThreads, smem, st>>>(*ex.g, *ex.w, counts);
     };
     // d <= 4 comes here from single calls only
@@ -68,7 +69,7 @@ void launch_update_wide(const Exec& ex, int* counts, cudaStream_t st) {
             return;
         }
         const size_t smem = smem_of(lm);
-        if (smem > 36 * 1024) cudaFuncSetAttribute(batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 36 * 1024) EGG_CHECK(cudaFuncSetAttribute(batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         batch<<<ex.blocks(kShapeWide, kWideThreads), kWideThreads, smem, st>>>(ex.args(kShapeWide));
     };
     // Every grid of 4 < d <= 16 has keys (16 bits a dimension hold any width), so
