@@ -28,6 +28,7 @@
 // first ten iterations, 1M x 3D 60 -> 40 ms, 250k x 3D 23.0 -> 15.0,
 // 45,781 x 3D 9.5 -> 4.7, 100k x 4D 17.9 -> 8.2 ms, all bit-identical.
 #include <climits>
+#include <type_traits>
 
 #include "egg_common.cuh"
 #include "egg_host_common.h"
@@ -303,10 +304,12 @@ constexpr int kRowBlocks = 148 * 5;
 constexpr int kRowsAhead = 4;  // rows whose loads are in flight together
 
 // shared memory of one warp, in 16-byte words: its joint box, 32 cell records (key, first
-// point, points | box | sums), then 32 points (coordinates | sums)
+// point, points | box | sums), then 32 points (coordinates | sums); one dimension: 32 group records
 __host__ __device__ constexpr int cell_words(int d) { return 1 + 2 * pack_w(d) + pack_s(d); }
 __host__ __device__ constexpr int box_words(int d) { return (4 * (5 * d + 2) + 15) / 16; }
-__host__ __device__ constexpr int warp_words(int d) { return box_words(d) + 32 * cell_words(d) + 32 * (pack_w(d) + pack_s(d)); }
+__host__ __device__ constexpr int warp_words(int d) {
+    return box_words(d) + 32 * cell_words(d) + 32 * (pack_w(d) + pack_s(d)) + (d == 1 ? 32 * (pack_s(d) + 2 * pack_w(d)) : 0);
+}
 
 // float order as unsigned order, and back
 __device__ __forceinline__ unsigned order_key(float x) {
@@ -317,6 +320,16 @@ __device__ __forceinline__ float order_val(unsigned k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+// what the screening of candidates needs of the warp's joint box: the same for
+// all lanes, so it waits in shared memory (volatile: read where it is used)
+// instead of in every lane's registers
+template <int D>
+struct WarpBox {
+    int lo[D], hi[D], wide[D];
+    float xl[D], xh[D];
+    float mar, r2;
+};
+
 // One kept cell for the 32 lanes; a lane whose column is off (col.sm infinite)
 // contributes nothing.  A group of points that some lane has to walk is
 // brought into shared memory by the whole warp (one coalesced load per record
@@ -325,7 +338,8 @@ __device__ __forceinline__ float order_val(unsigned k) {
 template <int D, int OD>
 __device__ __forceinline__ void visit_cell_warp(const Geom& g, const Work& w, const ulonglong2* rec, const float* x,
                                                 const unsigned long long* nx, const int* gi, const Col<D>& col,
-                                                Acc<D>& a, const float4* tab, int K, ulonglong2* stage, int lane) {
+                                                Acc<D>& a, const float4* tab, int K, const volatile WarpBox<D>& B,
+                                                ulonglong2* stage, int lane) {
     constexpr int PW = pack_w(D), PS = pack_s(D);
     const int od = OD > 0 ? OD : g.od;
     const ulonglong2 head = rec[0];
@@ -365,24 +379,25 @@ __device__ __forceinline__ void visit_cell_warp(const Geom& g, const Work& w, co
     if (__any_sync(0xffffffffu, straddle)) {
         const int qe = qb + m_all;
         const int kh = qb >> 5, kt = (qe - 1) >> 5;
-        for (int k = kh; k <= kt; k++) {
+        // points of group k; gr: its record (several groups only)
+        auto visit_group = [&](int k, auto from, const ulonglong2* gr) {
+            constexpr bool kGlobal = decltype(from)::value;
             const int sb = max(qb, k << 5), se = min(qe, (k << 5) + 32);
             const int m = se - sb;
             bool walk = straddle;
             if (kh != kt) {
-                const ulonglong2* gr = reinterpret_cast<const ulonglong2*>(group_rec<D>(w, k, (k == kh) ? 1 : 0, D));
                 float n2, f2;
-                box_dist2<D, true>(nx, x, gr + PS, n2, f2);
+                box_dist2<D, kGlobal>(nx, x, gr + PS, n2, f2);
                 const bool g_in = straddle && !(n2 > g.t_eps) && f2 <= g.t_eps;
                 walk = straddle && !(n2 > g.t_eps) && !g_in;
                 EGG_STAT(a, kUsGroupsOut, straddle && n2 > g.t_eps);
                 EGG_STAT(a, kUsGroupsIn, g_in);
                 if (g_in) {
-                    add_point<D, true>(av, gr);
+                    add_point<D, kGlobal>(av, gr);
                     cnt += m;
                 }
             }
-            if (!__any_sync(0xffffffffu, walk)) continue;
+            if (!__any_sync(0xffffffffu, walk)) return;
             __syncwarp();
             if (lane < m) {
                 const ulonglong2* xp = reinterpret_cast<const ulonglong2*>(w.xp) + (size_t)(sb + lane) * PW;
@@ -409,6 +424,46 @@ __device__ __forceinline__ void visit_cell_warp(const Geom& g, const Work& w, co
                     }
                 }
             }
+        };
+        auto group = [&](int k) {
+            return reinterpret_cast<const ulonglong2*>(group_rec<D>(w, k, (k == kh) ? 1 : 0, D));
+        };
+        if constexpr (D == 1) {
+            // One dimension: cells of thousands of points.  Their groups come 32
+            // at a time, one per lane, and stay where an active lane can count a
+            // point of theirs (the screening of cells below); one load for all
+            // lanes per group waited 600 cycles each (1M x 1 at eps 0.05, first
+            // iteration: 15.0 ms, 5.4 with the screening, 5.5 with a thread per
+            // point).
+            constexpr int GW = PS + 2 * PW;
+            ulonglong2* const recs = stage + 32 * (PW + PS);
+            for (int k0 = kh; k0 <= kt; k0 += 32) {
+                bool keep = k0 + lane <= kt;
+                ulonglong2 r[GW];
+                if (keep && kh != kt) {
+                    const ulonglong2* gr = group(k0 + lane);
+#pragma unroll
+                    for (int j = 0; j < GW; j++) r[j] = __ldg(gr + j);
+                    float lo, hi, skip;
+                    unpack2(r[PS].x, lo, skip);
+                    unpack2(r[PS + PW].x, hi, skip);
+                    const float gap = fmaxf(fmaxf(lo - B.xh[0], B.xl[0] - hi) - B.mar, 0.f);
+                    keep = !(gap * gap > g.t_eps * 1.0001f);
+                }
+                unsigned kept = __ballot_sync(0xffffffffu, keep);
+                __syncwarp();  // the last chunk's records are read
+                if (keep && kh != kt) {
+#pragma unroll
+                    for (int j = 0; j < GW; j++) recs[lane * GW + j] = r[j];
+                }
+                __syncwarp();
+                for (; kept; kept &= kept - 1) {
+                    const int src = __ffs(kept) - 1;
+                    visit_group(k0 + src, std::false_type{}, recs + src * GW);
+                }
+            }
+        } else {
+            for (int k = kh; k <= kt; k++) visit_group(k, std::true_type{}, group(k));
         }
         EGG_STAT(a, kUsPairsIn, in ? 0 : cnt);
     }
@@ -425,16 +480,6 @@ __device__ __forceinline__ void visit_cell_warp(const Geom& g, const Work& w, co
         if (!full) a.partial_in += cnt;
     }
 }
-
-// what the screening of candidates needs of the warp's joint box: the same for
-// all lanes, so it waits in shared memory (volatile: read where it is used)
-// instead of in every lane's registers
-template <int D>
-struct WarpBox {
-    int lo[D], hi[D], wide[D];
-    float xl[D], xh[D];
-    float mar, r2;
-};
 
 template <int D, int OD, bool tiled>
 __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const float* x, const int* gi, bool act,
@@ -637,7 +682,7 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
                     col.sm = on ? sm : INFINITY;
                     col.lg = lg;
                 }
-                visit_cell_warp<D, OD>(g, w, rec, x, nx, gi, col, a, tab, K, stage, lane);
+                visit_cell_warp<D, OD>(g, w, rec, x, nx, gi, col, a, tab, K, B, stage, lane);
 #ifdef EGG_UPDATE_STATS
                 if (lane == 0) {
                     a.st[kUsWarpVisits] += 1;
