@@ -270,12 +270,21 @@ __device__ __forceinline__ void negate_pairs(const float* x, unsigned long long*
 // them) cost a thirty-second of a visit.
 //
 // With the joint box too wide the walk does not pay and returns false before
-// any visit: for more than kUnionCols columns (points of an empty region), and
+// any visit: for more than kUnionCols columns (points of an empty region), in
+// tile order for too wide a joint region (kTileRoom), and
 // in storage order (tiled false) when the lanes lie in several columns or
 // spread over dimension od and more than kSpreadCells cells are around them
 // (consecutive points of sparse columns are dozens of cells apart there).
 // ---------------------------------------------------------------------------
 constexpr int kUnionCols = 1024;
+// In tile order a joint region of more than this many times one point's own
+// (the curve leaves a cluster, or crosses an empty region) is not walked
+// together either: few such warps, but thousands of candidates each held the
+// whole launch (1M x 2D, eps 0.002, first update: 5.3 ms, 1.3 with 8 to 512; a
+// run of 200k x 4D: 33.9 ms without, 48.3, 41.7, 37.7, 35.9, 34.0 and 34.0 with
+// 8, 16, 32, 64, 128 and 512; one of 43,110 x 3D, eps 0.00065: 6.5, 4.6 with
+// 128, 4.7 with 512).
+constexpr float kTileRoom = 128.f;
 // Whole rows of columns instead of columns where they hold at most this many
 // cells per column: once the points have gathered, nearly every column of the
 // hundreds around a warp is empty, and finding its few cells took 30 chained
@@ -493,7 +502,8 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
     int ncol;
     bool spread;  // storage order, several columns: only with few candidates in all
     {
-        float cols = 1.f, mar = 1.f;
+        float cols = 1.f, mar = 1.f, room = 1.f;
+        const float inv_reach = 1.0f / (float)(2 * g.r + 1);
         bool one = true;
 #pragma unroll
         for (int l = 0; l < D; l++) {
@@ -501,6 +511,7 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
             const int hi = __reduce_max_sync(0xffffffffu, act ? gi[l] : INT_MIN);
             const int wide = l < od ? min(g.width - 1, hi + g.r) - max(0, lo - g.r) + 1 : 1;
             cols *= (float)wide;
+            room *= 1.0f + (float)(hi - lo) * inv_reach;
             if (l < od) one = one && lo == hi;
             if (l == od) one = one && hi - lo <= kLockZSpan;
             // the active lanes' bounding box, and a margin for the rounding of
@@ -517,6 +528,7 @@ __device__ __forceinline__ bool walk_union(const Geom& g, const Work& w, const f
             }
         }
         if ((tiled || !one) && cols > (float)kUnionCols) return false;
+        if (tiled && room > kTileRoom) return false;
         spread = !tiled && !one;
         ncol = (int)cols;
         if (lane == 0) {
