@@ -695,17 +695,22 @@ def mdl_leg(dev):
 def run_reference(args, rank, world):
     """The reference's own CPU SynC on the box's host cores (rank 0 only):
     every step times one iteration of the same fixed sample as the
-    cpu_baseline leg and extrapolates to the whole run."""
+    cpu_baseline leg and extrapolates to the whole run.  Without its library
+    or its sources, a line that says so."""
     if rank != 0:
         return None
     sys.path.insert(0, str(REPO / "oracle"))
     from eggsync import data
     from oracle import RefSync
 
+    try:
+        R = RefSync()
+    except FileNotFoundError as e:
+        return {"impl": "reference",
+                "unavailable": "the reference's CPU SynC is not built here (%s)" % Path(str(e)).name}
     c = data.c5(args.seed, n=args.n)
     X, eps = c["X"], c["eps"]
     sample = args.cpu_sample or CPU_SAMPLE
-    R = RefSync()
     vals = []
     dts = []
     for k in range(args.warmup + args.steps):
