@@ -551,79 +551,40 @@ cudaGraphExec_t get_graph(State& S, Plan& P, const Config& c) {
             // [cell sums .. update, gate] -> IF(some instance flagged) [extra check]
             cudaGraph_t gbody = cp.conditional.phGraph_out[0];
             const Exec gex = batched(P.groups[k].act, P.groups[k].d);
-            cudaGraphNode_t prev = nullptr;  // last node so far (nullptr: none)
-            bool ok = true;
-            // capture `fn` into graph `into` after the dependency `dep`; its last node -> *last
+            cudaGraphNode_t prev = nullptr, ifs_sort = nullptr, ifs_tile = nullptr, ifs_x = nullptr;
+            cudaGraph_t sbody = nullptr, tbody = nullptr, xbody = nullptr;
+            auto then = [&](auto&& step) {
+                if (e == cudaSuccess) e = step();
+            };
             auto seg = [&](cudaGraph_t into, cudaGraphNode_t dep, cudaGraphNode_t* last, auto&& fn) {
-                cudaError_t r = cudaStreamBeginCaptureToGraph(S.st, into, dep ? &dep : nullptr, nullptr, dep ? 1 : 0,
-                                                              cudaStreamCaptureModeThreadLocal);
-                if (r != cudaSuccess) return r;
-                try {
-                    fn();
-                    if (last) {
-                        cudaStreamCaptureStatus cs;
-                        const cudaGraphNode_t* deps = nullptr;
-                        size_t nd = 0;
-                        EGG_CHECK(cudaStreamGetCaptureInfo(S.st, &cs, nullptr, nullptr, &deps, &nd));
-                        *last = nd == 1 ? deps[0] : nullptr;
-                    }
-                } catch (const CudaError& ce) {
-                    ok = false;
-                    r = ce.code;
-                }
-                cudaGraph_t captured = nullptr;
-                const cudaError_t r2 = cudaStreamEndCapture(S.st, &captured);
-                if (r == cudaSuccess) r = r2;
-                if (r == cudaSuccess && last && !*last) r = cudaErrorUnknown;
-                return r;
+                then([&] { return capture_into(S.st, into, dep, last, fn); });
             };
-            // an IF node in `into` after `dep` whose body `fill` captures; the node -> *node
-            auto cond = [&](cudaGraph_t into, cudaGraphConditionalHandle hc, cudaGraphNode_t dep, cudaGraphNode_t* node,
-                            auto&& fill) {
-                cudaGraphNodeParams xp = {cudaGraphNodeTypeConditional};
-                xp.conditional.handle = hc;
-                xp.conditional.type = cudaGraphCondTypeIf;
-                xp.conditional.size = 1;
-                cudaError_t r = cudaGraphAddNode(node, into, &dep, 1, &xp);
-                if (r == cudaSuccess) r = fill(xp.conditional.phGraph_out[0]);
-                return r;
-            };
-            auto cond_leaf = [&](cudaGraph_t into, cudaGraphConditionalHandle hc, cudaGraphNode_t dep,
-                                 cudaGraphNode_t* node, auto&& fn) {
-                return cond(into, hc, dep, node, [&](cudaGraph_t b) { return seg(b, nullptr, nullptr, fn); });
-            };
-            cudaGraphConditionalHandle hsort, hx;
-            e = cudaGraphConditionalHandleCreate(&hsort, gbody, 0, 0);
-            if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hx, gbody, 0, 0);
-            if (e == cudaSuccess)
-                e = seg(gbody, nullptr, &prev, [&] {
-                    enqueue_group(P, k, S.st, 0);
-                    launch_batch_gate_sort(gex, hsort, P.d_loop + 2 + k, S.st);
-                });
-            cudaGraphNode_t ifs_sort = nullptr, ifs_x = nullptr;
+            cudaGraphConditionalHandle hsort, ht, hx;
+            then([&] { return cudaGraphConditionalHandleCreate(&hsort, gbody, 0, 0); });
+            then([&] { return cudaGraphConditionalHandleCreate(&hx, gbody, 0, 0); });
+            seg(gbody, nullptr, &prev, [&] {
+                enqueue_group(P, k, S.st, 0);
+                launch_batch_gate_sort(gex, hsort, P.d_loop + 2 + k, S.st);
+            });
+            then([&] { return add_if_node(gbody, prev, hsort, &ifs_sort, &sbody); });
             // sort body: [sort, gate] -> IF(some instance wants a tile order) [tile order]
-            if (e == cudaSuccess)
-                e = cond(gbody, hsort, prev, &ifs_sort, [&](cudaGraph_t sb) {
-                    if (!gex.tile || gex.small_build()) return seg(sb, nullptr, nullptr, [&] { enqueue_group(P, k, S.st, 1); });
-                    cudaGraphConditionalHandle ht;
-                    cudaGraphNode_t last = nullptr, it_node = nullptr;
-                    cudaError_t r = cudaGraphConditionalHandleCreate(&ht, sb, 0, 0);
-                    if (r == cudaSuccess)
-                        r = seg(sb, nullptr, &last, [&] {
-                            enqueue_group(P, k, S.st, 1);
-                            launch_batch_gate_tile(gex, ht, P.d_loop + 2 + G + k, S.st);
-                        });
-                    if (r == cudaSuccess)
-                        r = cond_leaf(sb, ht, last, &it_node, [&] { enqueue_group(P, k, S.st, 4); });
-                    return r;
+            if (!gex.tile || gex.small_build()) {
+                seg(sbody, nullptr, nullptr, [&] { enqueue_group(P, k, S.st, 1); });
+            } else {
+                then([&] { return cudaGraphConditionalHandleCreate(&ht, sbody, 0, 0); });
+                seg(sbody, nullptr, &prev, [&] {
+                    enqueue_group(P, k, S.st, 1);
+                    launch_batch_gate_tile(gex, ht, P.d_loop + 2 + G + k, S.st);
                 });
-            if (e == cudaSuccess)
-                e = seg(gbody, ifs_sort, &prev, [&] {
-                    enqueue_group(P, k, S.st, 2);
-                    launch_batch_gate_extra(gex, hx, S.st);
-                });
-            if (e == cudaSuccess) e = cond_leaf(gbody, hx, prev, &ifs_x, [&] { enqueue_group(P, k, S.st, 3); });
-            if (!ok && e == cudaSuccess) e = cudaErrorUnknown;
+                then([&] { return add_if_node(sbody, prev, ht, &ifs_tile, &tbody); });
+                seg(tbody, nullptr, nullptr, [&] { enqueue_group(P, k, S.st, 4); });
+            }
+            seg(gbody, ifs_sort, &prev, [&] {
+                enqueue_group(P, k, S.st, 2);
+                launch_batch_gate_extra(gex, hx, S.st);
+            });
+            then([&] { return add_if_node(gbody, prev, hx, &ifs_x, &xbody); });
+            seg(xbody, nullptr, nullptr, [&] { enqueue_group(P, k, S.st, 3); });
         }
         if (e == cudaSuccess) {
             CtlArgs a = ctl_args(P);
@@ -638,19 +599,7 @@ cudaGraphExec_t get_graph(State& S, Plan& P, const Config& c) {
             e = cudaGraphAddKernelNode(&ctl, body, ifs.data(), G, &kp);
         }
     } else if (e == cudaSuccess) {
-        e = cudaStreamBeginCaptureToGraph(S.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            bool ok = true;
-            try {
-                enqueue_iteration(S, P, h, 1);
-            } catch (const CudaError& ce) {
-                ok = false;
-                e = ce.code;
-            }
-            cudaGraph_t captured = nullptr;
-            const cudaError_t e2 = cudaStreamEndCapture(S.st, &captured);
-            if (ok) e = e2;
-        }
+        e = capture_into(S.st, body, nullptr, nullptr, [&] { enqueue_iteration(S, P, h, 1); });
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);

@@ -34,6 +34,7 @@ namespace egg {
 
 std::mutex g_mutex;
 thread_local std::string g_last_error;
+int g_fail_captures = 0;  // injected capture failures still to deliver (egg_inject_capture_failures)
 int g_fail_allocs = 0;  // injected allocation failures still to deliver (egg_inject_alloc_failures)
 // interaction counters of the last run (stats build)
 unsigned long long g_counters[kUStats] = {};
@@ -307,7 +308,6 @@ struct Instance {
     // graph cache
     cudaGraphExec_t exec = nullptr;
     std::vector<char> graph_key;
-    bool graph_failed = false;
 };
 
 std::map<int, Instance*> g_inst;
@@ -516,116 +516,52 @@ bool ensure_graph(Instance& I) {
         e = cudaGraphAddNode(&node, graph, nullptr, 0, &p);
         if (e == cudaSuccess) body = p.conditional.phGraph_out[0];
     }
-    // body: [begin, grid check, gate] -> IF(changed) [grid sort] -> [rest of the iteration]
-    cudaGraphConditionalHandle hs;
-    cudaGraphNode_t tail = nullptr, ifnode = nullptr;
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hs, body, 1, 0);
-    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(I.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        enqueue_part(I, 0, h, 1);
-        k_gate_sort<<<1, 1, 0, I.st>>>(I.w, hs);
-        cudaStreamCaptureStatus cs;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t nd = 0;
-        e = cudaStreamGetCaptureInfo(I.st, &cs, nullptr, nullptr, &deps, &nd);
-        if (e == cudaSuccess && nd == 1) tail = deps[0];
-        cudaGraph_t captured = nullptr;
-        const cudaError_t e2 = cudaStreamEndCapture(I.st, &captured);
-        if (e == cudaSuccess) e = e2;
-        if (e == cudaSuccess && !tail) e = cudaErrorUnknown;
-    }
-    if (e == cudaSuccess) {
-        cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-        cp.conditional.handle = hs;
-        cp.conditional.type = cudaGraphCondTypeIf;
-        cp.conditional.size = 1;
-        e = cudaGraphAddNode(&ifnode, body, &tail, 1, &cp);
-        // sort body: [sort, gate] -> IF(the new grid wants a tile order) [tile order]
-        const bool tile = tile_capable(I.g) && I.w.bkey == nullptr;
-        cudaGraph_t sbody = nullptr;
-        cudaGraphConditionalHandle ht;
-        cudaGraphNode_t stail = nullptr;
-        if (e == cudaSuccess) sbody = cp.conditional.phGraph_out[0];
-        if (e == cudaSuccess && tile) e = cudaGraphConditionalHandleCreate(&ht, sbody, 0, 0);
-        if (e == cudaSuccess)
-            e = cudaStreamBeginCaptureToGraph(I.st, sbody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            enqueue_part(I, 1, h, 1);
-            if (tile) {
+    // body: [begin, grid check, gate] -> IF(changed) [grid sort] -> [rest of the
+    // iteration up to the update, gate] -> IF(flag) [extra check] -> [loop control];
+    // sort body: [sort, gate] -> IF(the new grid wants a tile order) [tile order]
+    cudaGraphConditionalHandle hs, ht, hx;
+    cudaGraph_t sbody = nullptr, tbody = nullptr, xbody = nullptr;
+    cudaGraphNode_t tail = nullptr, stail = nullptr, tail2 = nullptr, ifsort = nullptr, iftile = nullptr, ifx = nullptr;
+    auto then = [&](auto&& step) {
+        if (e == cudaSuccess) e = step();
+    };
+    const bool tile = tile_capable(I.g) && I.w.bkey == nullptr;
+    then([&] { return cudaGraphConditionalHandleCreate(&hs, body, 1, 0); });
+    then([&] {
+        return capture_into(I.st, body, nullptr, &tail, [&] {
+            enqueue_part(I, 0, h, 1);
+            k_gate_sort<<<1, 1, 0, I.st>>>(I.w, hs);
+        });
+    });
+    then([&] { return add_if_node(body, tail, hs, &ifsort, &sbody); });
+    if (tile) {
+        then([&] { return cudaGraphConditionalHandleCreate(&ht, sbody, 0, 0); });
+        then([&] {
+            return capture_into(I.st, sbody, nullptr, &stail, [&] {
+                enqueue_part(I, 1, h, 1);
                 k_gate_tile<<<1, 1, 0, I.st>>>(I.w, ht);
-                cudaStreamCaptureStatus cs;
-                const cudaGraphNode_t* deps = nullptr;
-                size_t nd = 0;
-                e = cudaStreamGetCaptureInfo(I.st, &cs, nullptr, nullptr, &deps, &nd);
-                if (e == cudaSuccess && nd == 1) stail = deps[0];
-            }
-            cudaGraph_t captured = nullptr;
-            const cudaError_t e2 = cudaStreamEndCapture(I.st, &captured);
-            if (e == cudaSuccess) e = e2;
-            if (e == cudaSuccess && tile && !stail) e = cudaErrorUnknown;
-        }
-        if (e == cudaSuccess && tile) {
-            cudaGraphNodeParams tp = {cudaGraphNodeTypeConditional};
-            tp.conditional.handle = ht;
-            tp.conditional.type = cudaGraphCondTypeIf;
-            tp.conditional.size = 1;
-            cudaGraphNode_t tnode = nullptr;
-            e = cudaGraphAddNode(&tnode, sbody, &stail, 1, &tp);
-            if (e == cudaSuccess)
-                e = cudaStreamBeginCaptureToGraph(I.st, tp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                  cudaStreamCaptureModeThreadLocal);
-            if (e == cudaSuccess) {
-                enqueue_part(I, 5, h, 1);
-                cudaGraph_t captured = nullptr;
-                e = cudaStreamEndCapture(I.st, &captured);
-            }
-        }
+            });
+        });
+        then([&] { return add_if_node(sbody, stail, ht, &iftile, &tbody); });
+        then([&] { return capture_into(I.st, tbody, nullptr, nullptr, [&] { enqueue_part(I, 5, h, 1); }); });
+    } else {
+        then([&] { return capture_into(I.st, sbody, nullptr, nullptr, [&] { enqueue_part(I, 1, h, 1); }); });
     }
-    // ... -> [rest of the iteration up to the update, gate] -> IF(flag) [extra check] -> [loop control]
-    cudaGraphConditionalHandle hx;
-    cudaGraphNode_t tail2 = nullptr, ifx = nullptr;
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hx, body, 0, 0);
-    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(I.st, body, &ifnode, nullptr, 1, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        enqueue_part(I, 2, h, 1);
-        launch_gate_extra(I.w, hx, I.st);
-        cudaStreamCaptureStatus cs;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t nd = 0;
-        e = cudaStreamGetCaptureInfo(I.st, &cs, nullptr, nullptr, &deps, &nd);
-        if (e == cudaSuccess && nd == 1) tail2 = deps[0];
-        cudaGraph_t captured = nullptr;
-        const cudaError_t e2 = cudaStreamEndCapture(I.st, &captured);
-        if (e == cudaSuccess) e = e2;
-        if (e == cudaSuccess && !tail2) e = cudaErrorUnknown;
-    }
-    if (e == cudaSuccess) {
-        cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-        cp.conditional.handle = hx;
-        cp.conditional.type = cudaGraphCondTypeIf;
-        cp.conditional.size = 1;
-        e = cudaGraphAddNode(&ifx, body, &tail2, 1, &cp);
-        if (e == cudaSuccess)
-            e = cudaStreamBeginCaptureToGraph(I.st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                              cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            enqueue_part(I, 3, h, 1);
-            cudaGraph_t captured = nullptr;
-            e = cudaStreamEndCapture(I.st, &captured);
-        }
-    }
-    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(I.st, body, &ifx, nullptr, 1, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        enqueue_part(I, 4, h, 1);
-        cudaGraph_t captured = nullptr;
-        e = cudaStreamEndCapture(I.st, &captured);
-    }
+    then([&] { return cudaGraphConditionalHandleCreate(&hx, body, 0, 0); });
+    then([&] {
+        return capture_into(I.st, body, ifsort, &tail2, [&] {
+            enqueue_part(I, 2, h, 1);
+            launch_gate_extra(I.w, hx, I.st);
+        });
+    });
+    then([&] { return add_if_node(body, tail2, hx, &ifx, &xbody); });
+    then([&] { return capture_into(I.st, xbody, nullptr, nullptr, [&] { enqueue_part(I, 3, h, 1); }); });
+    then([&] { return capture_into(I.st, body, ifx, nullptr, [&] { enqueue_part(I, 4, h, 1); }); });
     if (e == cudaSuccess) e = cudaGraphInstantiate(&I.exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
         cudaGetLastError();
         I.exec = nullptr;
-        I.graph_failed = true;
         return false;
     }
     I.graph_key = key;
@@ -1187,6 +1123,14 @@ __attribute__((visibility("default"))) int egg_inject_alloc_failures(int32_t cou
     return egg::guarded([&] {
         if (count < 0) throw egg::ArgError{EGG_ERR_ARG, "count must be >= 0"};
         egg::g_fail_allocs = count;
+        return (int)EGG_OK;
+    });
+}
+
+__attribute__((visibility("default"))) int egg_inject_capture_failures(int32_t count) {
+    return egg::guarded([&] {
+        if (count < 0) throw egg::ArgError{EGG_ERR_ARG, "count must be >= 0"};
+        egg::g_fail_captures = count;
         return (int)EGG_OK;
     });
 }

@@ -45,6 +45,53 @@ inline cudaError_t dev_alloc(void** p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
+// Captures what fn launches on st into the graph `into` after the node dep
+// (nullptr: no dependency); the last node -> *last (nullptr: not wanted).  A
+// failure in fn (a refused launch, an exception of EGG_CHECK) ends the capture
+// and is returned, so that the stream and the graph can be given up cleanly.
+// For tests, egg_inject_capture_failures(k) makes the next k captures fail.
+extern int g_fail_captures;
+template <typename F>
+cudaError_t capture_into(cudaStream_t st, cudaGraph_t into, cudaGraphNode_t dep, cudaGraphNode_t* last, F&& fn) {
+    EGG_CHECK(cudaPeekAtLastError());  // an earlier launch's error is the call's, not the capture's
+    cudaError_t r = cudaStreamBeginCaptureToGraph(st, into, dep ? &dep : nullptr, nullptr, dep ? 1 : 0,
+                                                  cudaStreamCaptureModeThreadLocal);
+    if (r != cudaSuccess) return r;
+    try {
+        if (g_fail_captures > 0) {
+            g_fail_captures--;
+            throw CudaError{cudaErrorInvalidConfiguration, "injected capture failure"};
+        }
+        fn();
+        r = cudaGetLastError();
+        if (r == cudaSuccess && last) {
+            cudaStreamCaptureStatus cs;
+            const cudaGraphNode_t* deps = nullptr;
+            size_t nd = 0;
+            r = cudaStreamGetCaptureInfo(st, &cs, nullptr, nullptr, &deps, &nd);
+            *last = r == cudaSuccess && nd == 1 ? deps[0] : nullptr;
+            if (r == cudaSuccess && !*last) r = cudaErrorUnknown;
+        }
+    } catch (const CudaError& ce) {
+        r = ce.code;
+    }
+    cudaGraph_t captured = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(st, &captured);
+    return r == cudaSuccess ? e : r;
+}
+
+// an IF node in `into` after dep, opened by hc; its body -> *body
+inline cudaError_t add_if_node(cudaGraph_t into, cudaGraphNode_t dep, cudaGraphConditionalHandle hc,
+                               cudaGraphNode_t* node, cudaGraph_t* body) {
+    cudaGraphNodeParams p = {cudaGraphNodeTypeConditional};
+    p.conditional.handle = hc;
+    p.conditional.type = cudaGraphCondTypeIf;
+    p.conditional.size = 1;
+    const cudaError_t r = cudaGraphAddNode(node, into, &dep, 1, &p);
+    if (r == cudaSuccess) *body = p.conditional.phGraph_out[0];
+    return r;
+}
+
 // geometry exactly as the reference computes it (EGG_SynC.cu:1249-1260, 1430, 563, 779, 1045)
 Geom make_geom(int64_t n64, int d, float eps);
 

@@ -292,6 +292,12 @@ int egg_abi_version(void);
  * EGG_ERR_ARG. */
 int egg_inject_alloc_failures(int32_t count);
 
+/* The same for the capture of a loop's CUDA graph: the next `count` captures
+ * of a part of it fail as a refused launch does.  The call then drives its
+ * loop from the host, with the same results, and the next call captures
+ * again.  A graph that is cached is not captured (egg_release() drops it). */
+int egg_inject_capture_failures(int32_t count);
+
 /* Interaction counters of the update kernel summed over the last
  * egg_sync_run: point updates computed, candidate cells examined, cells
  * passing the reference's small box test, cells aggregated as fully covered,
