@@ -21,6 +21,10 @@
 // single-instance wrapper and a batched wrapper (egg_batch.cuh).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+#include <map>
+#include <utility>
+
 #include "egg_common.cuh"
 #include "egg_host_common.h"
 #include "egg_kernels.h"
@@ -1396,26 +1400,55 @@ void launch_build(const Exec& ex, cudaStream_t st) {
     launch_build_sort(ex, st);
 }
 
-void launch_build_small(const Exec& ex, cudaStream_t st) {
-    const int C = small_cluster(ex.batch() ? ex.bt->max_n : ex.g->n);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = C;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ex.batch() ? C * ex.bt->instances : C);
-    cfg.blockDim = dim3(32 * kSmallWarps);
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    auto go = [&](auto one, auto batch) {
-        if (ex.batch()) {
-            if (C > 8) EGG_CHECK(cudaFuncSetAttribute(batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            EGG_CHECK(cudaLaunchKernelEx(&cfg, batch, ex.args(0)));
-        } else {
-            if (C > 8) EGG_CHECK(cudaFuncSetAttribute(one, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            EGG_CHECK(cudaLaunchKernelEx(&cfg, one, *ex.g, *ex.w));
+// The largest cluster of at most `want` blocks that this device can hold (16
+// are more than every device has to; fewer compute the same).  Asked once per
+// kernel and device, under the lock of the entry points.
+static int cluster_that_fits(const void* kernel, int want) {
+    static std::map<std::pair<int, const void*>, int> most;
+    int dev = 0;
+    EGG_CHECK(cudaGetDevice(&dev));
+    auto it = most.find({dev, kernel});
+    if (it == most.end()) {
+        int C = 16;
+        for (; C > 1; C /= 2) {
+            if (C > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+                cudaGetLastError();
+                continue;
+            }
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = C;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(C);
+            cfg.blockDim = dim3(32 * kSmallWarps);
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) break;
+            cudaGetLastError();
         }
+        it = most.emplace(std::make_pair(dev, kernel), C).first;
+    }
+    return std::min(want, it->second);
+}
+
+void launch_build_small(const Exec& ex, cudaStream_t st) {
+    auto go = [&](auto one, auto batch) {
+        const void* kernel = ex.batch() ? (const void*)batch : (const void*)one;
+        const int C = cluster_that_fits(kernel, small_cluster(ex.batch() ? ex.bt->max_n : ex.g->n));
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ex.batch() ? C * ex.bt->instances : C);
+        cfg.blockDim = dim3(32 * kSmallWarps);
+        cfg.stream = st;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        if (ex.batch()) EGG_CHECK(cudaLaunchKernelEx(&cfg, batch, ex.args(0)));
+        else EGG_CHECK(cudaLaunchKernelEx(&cfg, one, *ex.g, *ex.w));
     };
     switch (ex.d) {
         case 1: go(k_build_small<1>, kb_build_small<1>); break;
