@@ -126,6 +126,7 @@ struct Work {
     float* cbox;       // [ns][2 * box_w(d)] tight bounding box of the cell's points: lower, then upper corner
     int* outer_begin;  // [n_outer + 1]
     unsigned long long* colmask;  // [n_outer] per outer cell: the blocks of zblk cells of dimension od holding a cell
+                                  // (order parameter, od < d; nullptr otherwise)
     // scratch for scans / sorts
     int* hist;         // [256 * tiles]
     int* digit_total;  // [256]

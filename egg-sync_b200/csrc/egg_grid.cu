@@ -573,7 +573,7 @@ __device__ __forceinline__ void heads_finalize_body(const Geom& g, const Work& w
 }
 
 // outer_begin[o] = first cell whose outer id >= o, o in [0, n_outer]; with
-// od < d, colmask[o] = the blocks of dimension od (zblk cells each, bit
+// od < d and an order parameter, colmask[o] = the blocks of dimension od (zblk cells each, bit
 // z / zblk) that hold a cell of outer cell o
 __device__ __forceinline__ void outer_ranges_body(const Geom& g, const Work& w, int bx, int gx) {
     EGG_SKIP_IF_UNCHANGED(w.ctrl);

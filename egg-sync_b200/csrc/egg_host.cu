@@ -191,7 +191,9 @@ size_t layout_work(const Geom& g, int max_iter, char* base, Work& w, float** xin
     add((void**)&w.csum, 4 * (size_t)sum_w(d) * ns);
     add((void**)&w.cbox, 4 * 2 * (size_t)box_w(d) * ns);
     add((void**)&w.outer_begin, 4 * ((size_t)g.n_outer + 1));
-    add((void**)&w.colmask, g.od < d ? 8 * ((size_t)g.n_outer + 1) : 0);
+    const bool cols = g.od < d && g.order_mode != 0;  // read by the order parameter alone
+    add((void**)&w.colmask, cols ? 8 * ((size_t)g.n_outer + 1) : 0);
+    if (!cols) w.colmask = nullptr;
     add((void**)&w.hist, 4 * 256 * (size_t)tiles);
     add((void**)&w.digit_total, 4 * 256);
     add((void**)&w.block_sums, 4 * (size_t)nb);

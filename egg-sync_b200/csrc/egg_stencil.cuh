@@ -1,4 +1,5 @@
-// egg_stencil.cuh -- candidate-cell enumeration shared by the per-point kernels.
+// egg_stencil.cuh -- candidate-cell enumeration of the order parameter (the
+// update walks its candidates itself, egg_update.cu and egg_point_walk.cuh).
 //
 // For a point with cell dims gi (outer id obase) the candidate cells are the
 // inner cells of the outer cells in the box stencil [-r, r]^od (the
@@ -16,15 +17,7 @@
 // Both paths give every lane the same results bit for bit: the extra cells
 // of the union fail that lane's box test.
 // fn(c) is called once per candidate cell per lane, in increasing stencil
-// entry then increasing cell order in both paths.  col(s) is called before
-// the cells of stencil entry s (whole outer columns: every cell of one shares
-// its coordinates in the outer dimensions); a lane for which it returns false
-// needs no cell of that column.  Lockstep visits a column unless every lane
-// passes it over; a lane's own walk does not look the column up at all.
-// A lane for which
-// active() is false needs no result: it rides along in the lockstep path
-// and skips its own walk in the other (active() is evaluated there only, so
-// the lockstep path carries nothing extra).
+// entry then increasing cell order in both paths.
 //
 // In a lane's own walk with od < d, an outer cell none of whose blocks of
 // dimension od (colmask) meets the lane's z-window holds no candidate: it is
@@ -38,7 +31,6 @@
 namespace egg {
 
 // warps whose cells in dimension od span more than this take the per-lane walk
-// (1M x 3D: 96.4 -> 95.5 ms against lockstep for every single-column warp)
 constexpr int kLockZSpan = 4;
 
 // colmask bits of the blocks meeting the cells [zl, zh] of dimension od
@@ -47,9 +39,9 @@ __device__ __forceinline__ unsigned long long zwindow_mask(const Geom& g, int zl
     return (2ull << bh) - (1ull << bl);  // bits bl..bh (bh = 63 wraps to the right value)
 }
 
-template <typename A, typename C, typename F>
+template <typename F>
 __device__ __forceinline__ void for_candidates(const Geom& g, const Work& w, const int* gi, int obase, int lane,
-                                               int d, A&& active, C&& col, F&& fn) {
+                                               int d, F&& fn) {
     const int nst = w.st_count[0];
     const int ob0 = __shfl_sync(0xffffffffu, obase, 0);
     int zlo = 0, zhi = 0;
@@ -84,12 +76,10 @@ __device__ __forceinline__ void for_candidates(const Geom& g, const Work& w, con
                 live &= live - 1;
                 const int b = __shfl_sync(0xffffffffu, cb, src);
                 const int e = __shfl_sync(0xffffffffu, ce, src);
-                if (!__any_sync(0xffffffffu, col(s0 + src))) continue;
                 for (int c = b; c < e; c++) fn(c);
             }
         }
     } else {
-        if (!active()) return;  // no warp-wide operation below
         // each lane walks its own stencil; the column masks of four entries
         // are loaded together, so most columns cost a quarter of a load
         constexpr int kAhead = 4;
@@ -115,7 +105,7 @@ __device__ __forceinline__ void for_candidates(const Geom& g, const Work& w, con
 #pragma unroll 1
             for (int k = 0; k < kAhead; k++) {
                 const int o = ol[k];
-                if (o < 0 || !col(s0 + k)) continue;
+                if (o < 0) continue;
                 int cb = __ldg(w.outer_begin + o), ce = __ldg(w.outer_begin + o + 1);
                 if (cb >= ce) continue;
                 if (g.od < d) {
