@@ -399,8 +399,8 @@ def update_fp32_leg(args, update_ms):
     return {"bound": "fp32", "kernel": "k_update", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
             "frac": ach / peak, "peak_source": "nominal (148 SMs x 128 FP32 lanes x 2 x 1965 MHz)",
             "algorithmic_flops": flops, "counters": k,
-            "note": "issue-bound, not FP32-bound: warp-issue and lane-activity figures from ncu in "
-                    "profiles/k_update_c5_1M.md"}
+            "note": "bound by issue and latency, not by FP32: pairs / (32 x walk_steps) is the share of lanes at work "
+                    "in the point walks; warp-issue figures from ncu in profiles/k_update_c5_1M.md"}
 
 
 def cpu_sample_idx(n, sample):

@@ -209,11 +209,11 @@ enum : int {
     kUsGroupsOut,      // 32-point groups skipped
     kUsPairs,          // point-pair distance tests
     kUsPairsIn,        // ... within eps
-    kUsLaneWarps,      // warps whose lanes span several outer cells
+    kUsLaneWarps,      // warps with points left to be walked one by one
     kUsHalfCount,      // border points that needed the half count
     kUsNeighbors,      // sum of |N(p)|
-    kUsCyclesShared,   // SM cycles of the candidate walk, warps whose lanes share one outer cell
-    kUsCyclesLane,     // SM cycles of the candidate walk, warps whose lanes span several outer cells
+    kUsCyclesShared,   // SM cycles of the joint candidate walk, warps that settle all their points so
+    kUsCyclesLane,     // ... the other warps (their single points' walks not included)
     kUsWarpVisits,     // candidate cells visited by lockstep warps (once per warp)
     kUsCyclesVisits,   // SM cycles of those visits (box tests, aggregates, walks): the rest of
                        // cycles_shared is the stencil enumeration

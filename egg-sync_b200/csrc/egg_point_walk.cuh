@@ -255,6 +255,7 @@ __device__ __forceinline__ void walk_point(const Geom& g, const Work& w, const f
 #pragma unroll
                                 for (int l = 0; l < 2 * LM; l++) av[l] += v[l];
                                 cnt++;
+                                EGG_WSTAT(kUsPairsIn, 1);
                             }
                         } else {
 #pragma unroll U
@@ -274,11 +275,11 @@ __device__ __forceinline__ void walk_point(const Geom& g, const Work& w, const f
                                     am[l] += __ldg(sm + l * step);
                                 }
                                 cnt++;
+                                EGG_WSTAT(kUsPairsIn, 1);
                             }
                         }
                     }
                 }
-                EGG_WSTAT(kUsPairsIn, cnt);
             }
         }
         const unsigned mask = __ballot_sync(0xffffffffu, cnt > 0);

@@ -430,6 +430,7 @@ __device__ __forceinline__ void visit_cell_warp(const Geom& g, const Work& w, co
                     if (pair_dist2<D>(stage + j * PW, nx, x) <= g.t_eps) {
                         add_point<D, false>(av, stage + 32 * PW + j * PS);
                         cnt++;
+                        EGG_STAT(a, kUsPairsIn, 1);
                     }
                 }
             }
@@ -474,7 +475,6 @@ __device__ __forceinline__ void visit_cell_warp(const Geom& g, const Work& w, co
         } else {
             for (int k = kh; k <= kt; k++) visit_group(k, std::true_type{}, group(k));
         }
-        EGG_STAT(a, kUsPairsIn, in ? 0 : cnt);
     }
     if (cnt) {
         float v[4 * PS];

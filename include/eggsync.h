@@ -303,9 +303,9 @@ int egg_inject_capture_failures(int32_t count);
  * passing the reference's small box test, cells aggregated as fully covered,
  * cells aggregated / skipped by their points' tight box, 32-point groups
  * aggregated / skipped, point-pair distance tests, pairs within eps, warps
- * that walked the stencil lane by lane, half-count evaluations, sum of
- * |N(p)|, SM cycles of the candidate walk in warps whose lanes share one
- * outer cell and in warps that walked lane by lane (in this order; 16
+ * with points left to be walked one by one, half-count evaluations, sum of
+ * |N(p)|, SM cycles of the joint candidate walk in warps that settle all
+ * their points so and in the others (in this order; 16
  * slots).  Only the stats build
  * (libeggsync_stats.so) collects them; it writes min(cap, 16) values and
  * returns 16.  The normal build returns 0.  No counterpart in the reference. */
