@@ -872,14 +872,15 @@ Config autotune(State& S, Plan& P) {
     auto trial2 = [&](const Config& c) { return std::min(time_trial(S, P, c), time_trial(S, P, c)); };
     float tb = trial2(best);
     // The trials see the first iterations only, where nearly every point is
-    // recomputed; what the many that follow want differs from sweep to sweep (48
-    // instances of up to 68,535 points: 69.3 ms with blocks of 256, 72.1 with 128;
-    // 144 two-dimensional ones of up to 179,575: 183 and 175; the first with 8
-    // blocks per SM 72, with 16, a little ahead in the trials, 75), so another
-    // size or number of blocks has to be 5% ahead.
+    // recomputed; what the many that follow want differs from sweep to sweep.
+    // Blocks of another size have to be 5% ahead (48 instances of up to 68,535
+    // points: 69.3 ms with 256 threads, 72.1 with 128; 144 two-dimensional ones
+    // of up to 179,575: 183 and 175), another number of them 6% (the first sweep
+    // loses 3% to 16 per SM, 1% to 6% ahead in the trials; all 512 instances of
+    // up to 179,575 points gain 3% from it, 7% ahead).
     auto consider = [&](Config c) {
         const float t = trial2(c);
-        if (t < tb * (c.update_threads != best.update_threads || c.occ != best.occ ? 0.95f : 1.0f)) {
+        if (t < tb * (c.update_threads != best.update_threads ? 0.95f : c.occ != best.occ ? 0.94f : 1.0f)) {
             tb = t;
             best = c;
         }
